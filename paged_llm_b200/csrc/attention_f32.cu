@@ -5,24 +5,64 @@
 
 constexpr int F32_ROWS = 16;     // query rows per block
 constexpr int F32_KEYS = 32;     // keys per iteration: one per lane
-constexpr int F32_MAXD = 256;
+constexpr int F32_STAGES = 2;
 
-// grid: (items, kv heads); 128 threads = 4 warps, each owning 4 of the 16 rows.
+__device__ __forceinline__ void f32_copy(float* dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
+}
+
+// grid: (items, kv heads); 128 threads = 4 warps, each owning 4 of the 16 rows.  A tile of 32 keys is brought in by
+// 16-byte asynchronous copies while the one before is worked on; the 32 keys' addresses are looked up a tile earlier
+// still.  What bounds it is the issue of shared-memory loads, so four rows share each: a lane reads four elements of
+// its key for four rows' dot products, and the four rows' probabilities of a key as one float4 for its two columns of
+// the weighted sum.  Every sum keeps its order (over the head's elements, over the keys).
+// NC: pairs of columns per lane, ceil(d / 64).
+template <int NC>
 __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     attn_zero_padding<float>(p);
     const AttnItem it = attn_decode_item(p, blockIdx.x / p.nkv, F32_ROWS, F32_KEYS);
     if (!it.valid) return;
-    extern __shared__ float smem[];
-    const int d = p.d, kvh = blockIdx.x % p.nkv, G = p.nh / p.nkv;
-    float* Qs = smem;                          // [16][d]
-    float* Ks = Qs + F32_ROWS * d;             // [32][d + 1]
-    float* Vs = Ks + F32_KEYS * (d + 1);       // [32][d]
-    float* Ps = Vs + F32_KEYS * d;             // [4][32]
+    extern __shared__ __align__(16) float smem[];
+    __shared__ const float* rows[F32_STAGES][F32_KEYS];   // each key of a tile: its address, or null (nothing there)
+    const int d = p.d, kvh = blockIdx.x % p.nkv, G = p.nh / p.nkv, KP = d + 4;
+    float* Qs = smem;                                 // [16][d]
+    float* Ps = Qs + F32_ROWS * d;                    // [4 warps][32 keys][4 rows]
+    float* Ks = Ps + 4 * F32_KEYS * 4;                // [2][32][d + 4]: four words of padding, no bank conflicts
+    float* Vs = Ks + F32_STAGES * F32_KEYS * KP;      // [2][32][d]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* q = (const float*)p.q;
     const float* kv = (const float*)p.kv;
     const int* bt = p.block_table + (size_t)it.seq * p.bt_stride;
+    const int n_tiles = (it.key_hi - it.key_lo + F32_KEYS - 1) / F32_KEYS;
+    const size_t v_off = (size_t)p.nkv * p.ps * d;
 
+    auto find_rows = [&](int t) {                     // threads 0..31
+        int n = it.key_lo + t * F32_KEYS + tid;
+        const float* src = nullptr;
+        if (n < it.key_hi) {
+            if (n >= p.keep_first) n += it.gap;
+            const int page = bt[n / p.ps];            // (ps_shift is for the bfloat16 kernels)
+            if (page >= 0) src = kv + ((((size_t)page * 2) * p.nkv + kvh) * p.ps + n % p.ps) * d;
+        }
+        rows[t % F32_STAGES][tid] = src;
+    };
+    auto load_tile = [&](int t) {
+        const int st = t % F32_STAGES, chunks = d / 4;
+        float* kd = Ks + st * F32_KEYS * KP;
+        float* vd = Vs + st * F32_KEYS * d;
+        for (int e = tid; e < F32_KEYS * chunks; e += 128) {
+            const int j = e / chunks, c = (e - j * chunks) * 4;
+            const float* src = rows[st][j];
+            f32_copy(kd + j * KP + c, src != nullptr ? src + c : kv, src != nullptr ? 16 : 0);
+            f32_copy(vd + j * d + c, src != nullptr ? src + v_off + c : kv, src != nullptr ? 16 : 0);
+        }
+    };
+    if (tid < F32_KEYS) {
+        find_rows(0);
+        find_rows(1);
+    }
     for (int e = tid; e < F32_ROWS * d; e += 128) {
         const int r = e / d, c = e - r * d;
         const int R = it.row_base + r;
@@ -31,7 +71,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
         Qs[e] = v;
     }
     int pos[4], first[4];
-    float m[4], l[4], acc[4][F32_MAXD / 32], slope[4];
+    float m[4], l[4], acc[4][2 * NC], slope[4];
     const float* brow[4];
 #pragma unroll
     for (int rr = 0; rr < 4; ++rr) {
@@ -43,58 +83,89 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
         m[rr] = -INFINITY;
         l[rr] = 0.f;
 #pragma unroll
-        for (int cc = 0; cc < F32_MAXD / 32; ++cc) acc[rr][cc] = 0.f;
+        for (int cc = 0; cc < 2 * NC; ++cc) acc[rr][cc] = 0.f;
     }
-    const int ncc = (d + 31) / 32;
+    __syncthreads();
+    if (n_tiles > 0) load_tile(0);
+    asm volatile("cp.async.commit_group;\n" ::);
 
-    for (int kt = it.key_lo; kt < it.key_hi; kt += F32_KEYS) {
+    for (int t = 0; t < n_tiles; ++t) {
+        if (t + 1 < n_tiles) load_tile(t + 1);
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        for (int e = tid; e < F32_KEYS * d; e += 128) {
-            const int j = e / d, c = e - j * d;
-            int n = kt + j;
-            float kk = 0.f, vv = 0.f;
-            if (n < it.key_hi) {
-                if (n >= p.keep_first) n += it.gap;
-                const int page = bt[n / p.ps];      // (ps_shift is for the bfloat16 kernels)
-                if (page >= 0) {
-                    const size_t base = ((((size_t)page * 2) * p.nkv + kvh) * p.ps + n % p.ps) * d + c;
-                    kk = kv[base];
-                    vv = kv[base + (size_t)p.nkv * p.ps * d];
+        if (t + 2 < n_tiles && tid < F32_KEYS) find_rows(t + 2);      // the tile at hand no longer needs its addresses
+        const int st = t % F32_STAGES;
+        const int place = it.key_lo + t * F32_KEYS + lane, n = place + (place >= p.keep_first ? it.gap : 0);
+        if (pos[0] >= 0) {                                            // (a warp's rows beyond the last come last)
+            const float4* kr = reinterpret_cast<const float4*>(Ks + (st * F32_KEYS + lane) * KP);
+            const float4* qr = reinterpret_cast<const float4*>(Qs + warp * 4 * d);
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (int c = 0; c < d / 4; ++c) {
+                const float4 k4 = kr[c];
+#pragma unroll
+                for (int rr = 0; rr < 4; ++rr) {
+                    const float4 q4 = qr[rr * (d / 4) + c];
+                    s[rr] = fmaf(q4.x, k4.x, s[rr]);
+                    s[rr] = fmaf(q4.y, k4.y, s[rr]);
+                    s[rr] = fmaf(q4.z, k4.z, s[rr]);
+                    s[rr] = fmaf(q4.w, k4.w, s[rr]);
                 }
             }
-            Ks[j * (d + 1) + c] = kk;
-            Vs[j * d + c] = vv;
-        }
-        __syncthreads();
-        const int place = kt + lane, n = place + (place >= p.keep_first ? it.gap : 0);
+            float pj[4];
+            unsigned live = 0u;                                       // rows that see a key of this tile (uniform per warp)
 #pragma unroll
-        for (int rr = 0; rr < 4; ++rr) {
-            if (pos[rr] < 0) continue;                   // uniform per warp
-            const float* qr = Qs + (warp * 4 + rr) * d;
-            const float* kr = Ks + lane * (d + 1);
-            float s = 0.f;
-            for (int c = 0; c < d; ++c) s = fmaf(qr[c], kr[c], s);
-            s = attn_score(p, s, slope[rr], n, pos[rr], brow[rr]);
-            const bool vis = place < it.key_hi && n <= pos[rr] && (n >= first[rr] || n < p.keep_first);
-            const float m_new = fmaxf(m[rr], warp_max(vis ? s : -INFINITY));
-            if (m_new == -INFINITY) continue;
-            const float pj = vis ? expf(s - m_new) : 0.f;
-            const float alpha = m[rr] == -INFINITY ? 0.f : expf(m[rr] - m_new);
-            l[rr] = l[rr] * alpha + warp_sum(pj);
-            m[rr] = m_new;
-            Ps[warp * 32 + lane] = pj;
+            for (int rr = 0; rr < 4; ++rr) {
+                pj[rr] = 0.f;
+                if (pos[rr] < 0) continue;                            // uniform per warp
+                const float sc = attn_score(p, s[rr], slope[rr], n, pos[rr], brow[rr]);
+                const bool vis = place < it.key_hi && n <= pos[rr] && (n >= first[rr] || n < p.keep_first);
+                const float m_new = fmaxf(m[rr], warp_max(vis ? sc : -INFINITY));
+                if (m_new == -INFINITY) continue;
+                if (__any_sync(0xffffffffu, vis)) live |= 1u << rr;
+                pj[rr] = vis ? expf(sc - m_new) : 0.f;
+                const float alpha = m[rr] == -INFINITY ? 0.f : expf(m[rr] - m_new);
+                l[rr] = l[rr] * alpha + warp_sum(pj[rr]);
+                m[rr] = m_new;
+#pragma unroll
+                for (int cc = 0; cc < 2 * NC; ++cc) acc[rr][cc] *= alpha;
+            }
+            float4* ps = reinterpret_cast<float4*>(Ps) + warp * F32_KEYS;
+            ps[lane] = make_float4(pj[0], pj[1], pj[2], pj[3]);
             __syncwarp();
+            const float* vr = Vs + st * F32_KEYS * d + lane * 2;
+            auto weigh = [&](int rr, float w, const float2& v, int cc) {
+                acc[rr][2 * cc] = fmaf(w, v.x, acc[rr][2 * cc]);
+                acc[rr][2 * cc + 1] = fmaf(w, v.y, acc[rr][2 * cc + 1]);
+            };
+            if (live == 15u) {
+#pragma unroll 8
+                for (int j = 0; j < F32_KEYS; ++j) {
+                    const float4 w = ps[j];
 #pragma unroll
-            for (int cc = 0; cc < F32_MAXD / 32; ++cc) {
-                const int c = lane + 32 * cc;
-                if (cc < ncc && c < d) {
-                    float a = acc[rr][cc] * alpha;
-                    for (int j = 0; j < F32_KEYS; ++j) a = fmaf(Ps[warp * 32 + j], Vs[j * d + c], a);
-                    acc[rr][cc] = a;
+                    for (int cc = 0; cc < NC; ++cc) {
+                        if (lane * 2 + 64 * cc >= d) continue;
+                        const float2 v = *reinterpret_cast<const float2*>(vr + j * d + 64 * cc);
+                        weigh(0, w.x, v, cc), weigh(1, w.y, v, cc), weigh(2, w.z, v, cc), weigh(3, w.w, v, cc);
+                    }
+                }
+            } else {
+                // a row that sees no key of the tile takes no part (its zeros times a value that is not finite would be NaN)
+                for (int j = 0; j < F32_KEYS; ++j) {
+                    const float4 w = ps[j];
+#pragma unroll
+                    for (int cc = 0; cc < NC; ++cc) {
+                        if (lane * 2 + 64 * cc >= d) continue;
+                        const float2 v = *reinterpret_cast<const float2*>(vr + j * d + 64 * cc);
+                        if (live & 1) weigh(0, w.x, v, cc);
+                        if (live & 2) weigh(1, w.y, v, cc);
+                        if (live & 4) weigh(2, w.z, v, cc);
+                        if (live & 8) weigh(3, w.w, v, cc);
+                    }
                 }
             }
-            __syncwarp();
         }
+        __syncthreads();                                              // the stage may be filled again
     }
 
 #pragma unroll
@@ -102,25 +173,26 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
         if (pos[rr] < 0) continue;
         const int R = it.row_base + warp * 4 + rr;
         const int tok = R / G, head = kvh * G + R % G;
+        float* o;
+        float f = 1.f;
         if (it.splits <= 1) {
-            float* o = (float*)p.out + (size_t)(it.q0 + tok) * p.out_stride + head * d;
+            o = (float*)p.out + (size_t)(it.q0 + tok) * p.out_stride + head * d;
             const float lsum = l[rr] + attn_sink_term(p, head, m[rr]);
-            const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
-#pragma unroll
-            for (int cc = 0; cc < F32_MAXD / 32; ++cc) {
-                const int c = lane + 32 * cc;
-                if (cc < ncc && c < d) o[c] = acc[rr][cc] * inv;
-            }
+            f = lsum > 0.f ? 1.0f / lsum : 0.f;
         } else {
             float* part = attn_partial(p, it.scratch_base + tok, head, it.split);
             if (lane == 0) {
                 part[0] = m[rr];
                 part[1] = l[rr];
             }
+            o = part + 2;
+        }
 #pragma unroll
-            for (int cc = 0; cc < F32_MAXD / 32; ++cc) {
-                const int c = lane + 32 * cc;
-                if (cc < ncc && c < d) part[2 + c] = acc[rr][cc];
+        for (int cc = 0; cc < NC; ++cc) {
+            const int c = lane * 2 + 64 * cc;
+            if (c < d) {
+                o[c] = acc[rr][2 * cc] * f;
+                o[c + 1] = acc[rr][2 * cc + 1] * f;
             }
         }
     }
@@ -173,19 +245,24 @@ int pl_attn_check(const AttnParams& p, const char* who) {
     return 0;
 }
 
+template <int NC> static int launch_attn_f32(const AttnParams& p, cudaStream_t stream) {
+    const size_t smem = ((size_t)F32_ROWS * p.d + 4 * F32_KEYS * 4 + F32_STAGES * F32_KEYS * (2 * p.d + 4)) * sizeof(float);
+    constexpr size_t most = ((size_t)F32_ROWS * 64 * NC + 4 * F32_KEYS * 4 + F32_STAGES * F32_KEYS * (2 * 64 * NC + 4)) * sizeof(float);
+    static bool attr_set = false;
+    if (!attr_set) {
+        PL_CUDA(cudaFuncSetAttribute(attn_f32_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        attr_set = true;
+    }
+    PL_CUDA(launch_pdl(attn_f32_kernel<NC>, dim3(p.n_work * p.nkv), dim3(128), smem, stream, p));
+    return 0;
+}
+
 PL_EXPORT int pl_attention_f32(const AttnParams* params, cudaStream_t stream) {
     AttnParams p = *params;
     if (p.n_work == 0) return 0;
     if (int rc = pl_attn_check(p, "attention_f32")) return rc;
-    const size_t smem = ((size_t)F32_ROWS * p.d + F32_KEYS * (p.d + 1) + F32_KEYS * p.d + 4 * 32) * sizeof(float);
-    static bool attr_set = false;
-    if (!attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(attn_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-        attr_set = true;
-    }
-    attn_f32_kernel<<<dim3(p.n_work * p.nkv), 128, smem, stream>>>(p);
-    PL_LAUNCHED("attention_f32");
-    return 0;
+    PL_REQUIRE(((uintptr_t)p.kv & 15) == 0, "attention_f32: kv must be 16-byte aligned");
+    return p.d <= 64 ? launch_attn_f32<1>(p, stream) : p.d <= 128 ? launch_attn_f32<2>(p, stream) : launch_attn_f32<4>(p, stream);
 }
 
 PL_EXPORT int pl_attention_combine(const AttnParams* params, int out_dtype, cudaStream_t stream) {

@@ -79,6 +79,19 @@ def test_gemm_f32_is_true_float32_and_batch_independent(ops, M, N, K):
     assert torch.equal(one[0], out[M // 2]), "a row's product must not depend on the rows beside it"
 
 
+@pytest.mark.parametrize("N,K", [(65, 31), (130, 257), (64, 2048), (2049, 260), (33, 5632), (12000, 1024)])
+def test_gemm_f32_shapes_agree(ops, N, K):
+    """Every tile shape, both ways of taking the parts of k (cluster, one after the other) and both copy widths (rows of
+    K % 4 != 0 are not 16-byte aligned) give a row the same bits.  The sums are chains of at most 704 / 2 terms, then at most
+    eight: an error of sqrt(352 + 8) rounding steps of 2^-24 on terms of size sqrt(K) in all is 5 sigma below the bound."""
+    a, b = randn(600, K, seed=5), randn(N, K, seed=6)
+    want = a.double() @ b.double().T
+    full = ops.linear(a, b)
+    assert (full - want).abs().max().item() < 2 ** -24 * 19 * math.sqrt(K) * 5
+    for M in (1, 2, 3, 4, 5, 8, 9, 32, 33, 64, 65, 129):
+        assert torch.equal(ops.linear(a[:M].contiguous(), b), full[:M]), f"{M} rows"
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 509, 96), (70, 172, 64), (5, 64, 172), (2048, 256, 512)])
 def test_linear_bf16(ops, M, N, K):
     a, b = randn(M, K, seed=7, dtype=torch.bfloat16), randn(N, K, seed=8, dtype=torch.bfloat16)
