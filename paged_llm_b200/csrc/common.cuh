@@ -168,6 +168,8 @@ struct AttnParams {
     // With a window: > 0: the first `keep_first` keys of a request stay visible to every later query beside the window
     // (at their true positions).  Without a window it means nothing.
     int keep_first;
+    // Small items: no request brings more query rows per kv head than this (0: up to 16).
+    int small_rows;
 };
 
 // What the sink adds to a row's sum of exponentials taken relative to the maximum `m` (natural-log units; -inf:

@@ -52,6 +52,7 @@ class AttentionPlan:
     max_splits: int
     small_tokens: int = 0            # tokens of the requests in `small` (scratch rows)
     long_context: bool = False       # a decode step whose contexts are split through the work list, not as clusters
+    even: bool = False               # a step whose small items are cut into ranges of about equal length (work list)
 
 
 @dataclass

@@ -272,7 +272,8 @@ class ModelRunner:
                 small=view(f"small{key}", ns * 4).view(ns, 4) if ns else None,
                 large=view(f"large{key}", nl * 4).view(nl, 4) if nl else None,
                 splits=view(f"splits{key}"), n_small=ns, n_large=nl, max_splits=p["max_splits"],
-                small_tokens=p["num_small_tokens"], long_context=p.get("long_context", False))
+                small_tokens=p["num_small_tokens"], long_context=p.get("long_context", False),
+                even=p.get("even", False))
         return StepContext(
             ops=self.ops, num_tokens=T, num_seqs=S, num_logits=info["L_pad"],
             input_ids=view("ids"), positions=view("pos"), token_seq=view("tseq"), cu_seqlens_q=view("cu"),

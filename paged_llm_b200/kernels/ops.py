@@ -47,7 +47,7 @@ class AttnParams(ctypes.Structure):
         ("scale", c_float), ("ps_shift", c_int), ("counters", c_void_p), ("num_pages", c_int), ("cluster", c_int),
         ("softcap", c_float), ("slopes", c_void_p), ("rope_table", c_void_p), ("rope_len", c_int),
         ("pad_seqs", c_int), ("pad_to", c_int), ("chunk", c_int), ("dist_bias", c_void_p), ("dist_len", c_int),
-        ("sink", c_void_p), ("keep_first", c_int),
+        ("sink", c_void_p), ("keep_first", c_int), ("small_rows", c_int),
     ]
 
 
@@ -138,8 +138,6 @@ class CudaOps:
         self.cluster_attention = os.environ.get("PAGED_LLM_B200_NO_CLUSTER") is None   # decode attention as clusters
         # decode steps of more than 16 tokens: rotary positions and the cache write inside the attention kernel
         self.rope_in_attention = os.environ.get("PAGED_LLM_B200_NO_ROPE_IN_ATTENTION") is None
-        # long work-list ranges of decode attention in a ring of three 64-key tiles (head sizes up to 64)
-        self.deep_list = os.environ.get("PAGED_LLM_B200_NO_DEEP_LIST") is None
         # lanes that share a column of the delta rule's state (8 unless 16 or 32 is asked for, for measurements)
         self.delta_lanes = int(os.environ.get("PAGED_LLM_B200_DELTA_LANES", "0"))
         self._argmax_ws = None            # (packed winners, arrival counters) of the multi-block argmax
@@ -1263,7 +1261,13 @@ class CudaOps:
             large_rows=self._large_rows(head_dim), min_split_keys=self.MIN_SPLIT_KEYS, num_sms=self.num_sms,
             max_splits=self.MAX_SPLITS, pad_requests=pad_requests, fixed_capacity=fixed_capacity,
             cluster_max=self.MAX_CLUSTER if self.cluster_attention else 0, long_keys=self.CLUSTER_KEYS,
-            pad_tokens=pad_tokens)
+            pad_tokens=pad_tokens, slots=self._attention_slots(head_dim))
+
+    def _attention_slots(self, head_dim: int) -> int:
+        """Blocks of the decode kernel that are resident at a time, two per SM (0: its ranges are not cut evenly)."""
+        if self.compute_dtype != torch.bfloat16 or not self.cluster_attention:
+            return 0
+        return 2 * self.num_sms
 
     def _scratch_for(self, floats: int) -> torch.Tensor:
         """Scratch for split partials.  Grown by allocating anew and keeping the
@@ -1281,7 +1285,13 @@ class CudaOps:
         """Whether this step's attention takes the cluster form of the decode kernel: every request
         is a small item (a decode step), in bfloat16, with contexts short enough."""
         return bool(bf16 and self.cluster_attention and plan.n_small and not plan.n_large
-                    and max(ctx.host.q_lens) * (nh // nkv) <= self.SMALL_ROWS and not plan.long_context)
+                    and max(ctx.host.q_lens) * (nh // nkv) <= self.SMALL_ROWS and not plan.long_context
+                    and not plan.even)
+
+    @staticmethod
+    def _rotates_inside(plan, ctx) -> bool:
+        """A decode step whose ranges were cut evenly: the list form rotates and writes the cache as the clusters do."""
+        return bool(plan.even and plan.n_small and not plan.n_large and max(ctx.host.q_lens) == 1)
 
     def qkv_attention(self, h, w_qkv, nh, nkv, d, position, ctx, kv, block_table, scale, window, write=True,
                       softcap=None, slopes=None, chunk=None, value_from_key=False) -> torch.Tensor:
@@ -1296,7 +1306,8 @@ class CudaOps:
                   and not value_from_key
                   and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens
                   and not self._skinny_ok(h, (nh + 2 * nkv) * d) and self.compute_dtype == torch.bfloat16
-                  and kv.dtype == torch.bfloat16 and self._runs_as_clusters(plan, ctx, nh, nkv, True)
+                  and kv.dtype == torch.bfloat16
+                  and (self._runs_as_clusters(plan, ctx, nh, nkv, True) or self._rotates_inside(plan, ctx))
                   and self.rope_in_attention)
         if inside:
             qkv = self.linear(h, w_qkv)
@@ -1335,6 +1346,8 @@ class CudaOps:
         p.block_table, p.cu_q, p.k_lens = block_table.data_ptr(), ctx.cu_seqlens_q.data_ptr(), ctx.seq_lens_k.data_ptr()
         p.q_stride, p.out_stride, p.bt_stride = qkv.shape[1], nh * d, block_table.shape[1]
         p.nh, p.nkv, p.d, p.ps, p.num_pages = nh, nkv, d, kv.shape[3], kv.shape[0]
+        # (a step of mixed items may replay a graph in which later steps bring more tokens per small item)
+        p.small_rows = nh // nkv if max(ctx.host.q_lens) == 1 and not plan.n_large else self.SMALL_ROWS
         p.window, p.scale, p.max_splits = int(window or 0), float(scale), plan.max_splits
         p.softcap = float(softcap or 0.0)
         p.chunk, p.keep_first = int(chunk or 0), keep_first
@@ -1358,9 +1371,9 @@ class CudaOps:
             lib, fn = self.core, self.core.pl_attention_f32
         p.cluster = 0
         if rope is not None:
-            if not self._runs_as_clusters(plan, ctx, nh, nkv, bf16) or softcap or slopes is not None or dist_bias is not None or keep_first:
+            if not (bf16 and (self._runs_as_clusters(plan, ctx, nh, nkv, bf16) or self._rotates_inside(plan, ctx))) or softcap or slopes is not None or dist_bias is not None or keep_first:
                 raise KernelError("rotary positions inside the attention kernel: only for decode steps that run as "
-                                  "clusters, without score modifiers")
+                                  "clusters or in even ranges, without score modifiers")
             assert qkv.shape[1] == (nh + 2 * nkv) * d and rope.table.is_contiguous() and rope.rotary_dim == d
             p.rope_table, p.rope_len = rope.table.data_ptr(), rope.table.shape[0]
         if self._runs_as_clusters(plan, ctx, nh, nkv, bf16):
@@ -1375,10 +1388,7 @@ class CudaOps:
             floats = max(plan.small_tokens, 1) * nh * plan.max_splits * (d + 2)
             scratch = self._scratch_for(floats)
             p.scratch, p.scratch_floats = scratch.data_ptr(), scratch.numel()
-            # long ranges and blocks in plenty (two per SM or more): the ring of three 64-key tiles; with fewer
-            # blocks eight warps per block do better (one request x 16,384 keys: 1.00 against 1.10 ms per step)
-            deep = plan.long_context and self.deep_list and plan.n_small * nkv >= 2 * self.num_sms
-            p.work, p.n_work, p.is_small = plan.small.data_ptr(), plan.n_small, 2 if deep else 1
+            p.work, p.n_work, p.is_small = plan.small.data_ptr(), plan.n_small, 1
             fused_merge = bf16 and plan.max_splits > 1
             if fused_merge:
                 need = ctx.num_seqs * nkv

@@ -47,12 +47,75 @@ def is_long_context(num_requests: int, num_kv_heads: int, num_sms: int, max_spli
     return max_context > long_keys * cluster
 
 
+# What a block costs beside its keys (its start, its query, the merge of its warps), and what the merge of the ranges of a
+# request adds, in keys: 4 and 1.2 us where a block reads some 85 keys per us.
+BLOCK_KEYS, MERGE_KEYS = 350, 100
+
+
+def even_ranges(num_requests: int, num_kv_heads: int, num_sms: int, slots: int, max_splits: int) -> int:
+    """For a step whose small items are cut into ranges of about equal length (`split_evenly`): how many ranges per kv head
+    are resident at a time.  0: the step is not cut that way, since a block per request and kv head would leave SMs idle
+    and every request is split alike (the cluster form, which merges without global memory)."""
+    if slots <= 0 or wanted_splits(num_requests, num_kv_heads, num_sms, max_splits) > 1:
+        return 0
+    return max(1, slots // max(num_kv_heads, 1))
+
+
+def even_max_splits(scratch_rows: int, max_splits: int) -> int:
+    """Ranges a request may have in such a step: bounded so that the scratch for the partial results stays small (at 32
+    heads of 64 some 17 MB)."""
+    return int(max(4, min(max_splits, 2048 // max(scratch_rows, 1))))
+
+
+def split_evenly(keys: np.ndarray, extra: int, max_splits: int) -> np.ndarray:
+    """Ranges per request so that the blocks of a step end at about the same time although the requests' contexts differ
+    (131 to 3,500 keys in one batch: a block per request and kv head walks 3,500 keys alone while most others have long
+    ended).  `extra` ranges per kv head are resident at a time, and fit the lists beside one per request; of a few lengths
+    of a range, none below an even share, the one after which the last block should end first."""
+    total, longest = int(keys.sum()), int(keys.max())
+    share = max(128, -(-total // extra))
+    best = None
+    for length in [longest] + [int(share * f) for f in (1.0, 1.15, 1.35, 1.6, 2.0, 2.7, 4.0)]:
+        ns = np.clip(-(-keys // length), 1, max_splits)
+        cost = -(-keys // ns) + BLOCK_KEYS + MERGE_KEYS * (ns > 1)
+        # the last block ends no earlier than an even share, nor than k + 1 blocks of which a place must take that many
+        blocks = np.sort(np.repeat(cost, ns))[::-1]
+        at = blocks[::extra]
+        end = max(int(blocks.sum()) / extra, int((at * np.arange(1, len(at) + 1)).max()))
+        if best is None or end < best[0]:
+            best = (end, ns)
+    return best[1].astype(np.int32)
+
+
 def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_splits, fixed_capacity,
-                 cluster_max=0, long_keys=0) -> dict:
+                 cluster_max=0, long_keys=0, slots=0) -> dict:
     """The same plan for the common step in which every request brings one token, in array form."""
     n_req = S_pad if fixed_capacity else S
     long_context = is_long_context(n_req, num_kv_heads, num_sms, max_splits, cluster_max, long_keys,
                                    int(max(k_lens)) if len(k_lens) else 0)
+    extra = max(1, slots // max(num_kv_heads, 1)) if long_context and slots > 0 \
+        else even_ranges(n_req, num_kv_heads, num_sms, slots, max_splits)
+    if extra:
+        lk = np.asarray(k_lens, np.int64)
+        most = even_max_splits(n_req, max_splits)
+        ns = split_evenly(lk, extra, most)
+        order = np.argsort(-(lk // ns), kind="stable").astype(np.int32)          # long ranges first
+        many = ns[order]
+        first = np.cumsum(many) - many
+        total = int(ns.sum())
+        small = np.empty((total, 4), np.int32)
+        small[:, 0] = small[:, 1] = np.repeat(order, many)
+        small[:, 2] = np.arange(total, dtype=np.int32) - np.repeat(first, many).astype(np.int32)
+        small[:, 3] = np.repeat(many, many)
+        splits = np.ones((S_pad, 2), np.int32)
+        splits[:, 1] = 0
+        splits[:S, 0] = ns
+        splits[:S, 1] = np.arange(S, dtype=np.int32)
+        if fixed_capacity:
+            small = np.concatenate([small, np.full((S_pad + extra - total, 4), -1, np.int32)])
+        return {"small": small.reshape(-1), "large": np.zeros(0, np.int32), "splits": splits.reshape(-1),
+                "max_splits": int(most if fixed_capacity else ns.max()),
+                "num_small_tokens": int(S_pad if fixed_capacity else S), "long_context": long_context, "even": True}
     want = long_context_splits(n_req, num_kv_heads, num_sms, max_splits) if long_context \
         else wanted_splits(n_req, num_kv_heads, num_sms, max_splits)
     lk = np.asarray(k_lens, np.int64)
@@ -108,27 +171,36 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
                    large_rows: int, min_split_keys: int, num_sms: int, max_splits: int = 32,
                    pad_requests: int | None = None, fixed_capacity: bool = False, cluster_max: int = 0,
                    long_keys: int = 0, pad_tokens: int | None = None, chunk: int | None = None,
-                   keep_first: int | None = None) -> dict:
-    """`pad_tokens` (with `fixed_capacity`, for a step of mixed items that replays a captured graph): both lists
+                   keep_first: int | None = None, slots: int = 0) -> dict:
+    """`slots` > 0 (blocks that are resident at a time): steps of so many requests that none would be split, and
+    long-context steps, are cut into ranges of about equal length instead (see `split_evenly`).
+
+    `pad_tokens` (with `fixed_capacity`, for a step of mixed items that replays a captured graph): both lists
     get the capacity of any step of that many tokens and `pad_requests` requests, filled up with items of
     request -1 that the kernels skip."""
     S = len(q_lens)
     S_pad = pad_requests or S
     if pad_tokens is None and S and max(q_lens) == 1 and group_size <= small_rows and not window and not chunk:
         return _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_splits, fixed_capacity,
-                            cluster_max, long_keys)
+                            cluster_max, long_keys, slots)
     small_ids = [s for s in range(S) if q_lens[s] * group_size <= small_rows]
     n_small = S_pad if fixed_capacity else len(small_ids)
     want = wanted_splits(n_small, num_kv_heads, num_sms, max_splits)
+    cap = S_pad * want
+    # (what a captured graph has baked in depends on its capacity alone, also where no request is small this time)
+    extra = even_ranges(n_small, num_kv_heads, num_sms, slots, max_splits) if n_small else 0
+    if extra:
+        want = even_max_splits(S_pad * max(1, small_rows // group_size) if fixed_capacity else len(small_ids), max_splits)
+        cap = S_pad + extra
+    n_keys = [visible_keys(k_lens[s] - q_lens[s], k_lens[s], window, chunk, keep_first) for s in small_ids]
+    even = split_evenly(np.asarray(n_keys, np.int64), extra, want) if extra and small_ids else None
     splits = np.ones((S_pad, 2), np.int32)
     splits[:, 1] = 0
     small = []
     scratch_base = 0
-    for s in small_ids:
-        nq, lk = q_lens[s], k_lens[s]
-        first_pos = lk - nq
-        n_keys = visible_keys(first_pos, lk, window, chunk, keep_first)
-        ns = max(1, min(want, -(-n_keys // min_split_keys)))
+    for i, s in enumerate(small_ids):
+        nq = q_lens[s]
+        ns = int(even[i]) if extra else max(1, min(want, -(-n_keys[i] // min_split_keys)))
         splits[s] = (ns, scratch_base)
         for j in range(ns):
             small.append((s, scratch_base, j, ns))
@@ -143,9 +215,11 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
             last_tok = min(rows - 1, (t + 1) * large_rows - 1) // group_size
             large.append((k_lens[s] - q_lens[s] + last_tok, s, t))
     large.sort(key=lambda x: -x[0])                       # longest first
+    if even is not None:
+        length = {s: n // int(m) for s, n, m in zip(small_ids, n_keys, even)}
+        small.sort(key=lambda x: -length[x[0]])           # (stable: the ranges of a request stay side by side)
     small_arr = np.array(small, np.int32).reshape(-1, 4)
     if fixed_capacity:
-        cap = S_pad * want
         if len(small_arr) > cap:
             raise PlanCapacityError(f"{len(small_arr)} small items for a capacity of {cap}")
         pad = np.full((cap - len(small_arr), 4), -1, np.int32)
@@ -167,4 +241,5 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
         "max_splits": int(want),
         "num_small_tokens": small_tokens,
         "long_context": False,
+        "even": bool(extra),
     }

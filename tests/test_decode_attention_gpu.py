@@ -1,0 +1,81 @@
+"""Decode attention whose ranges are cut evenly (work list), with the rotation and the cache write inside, against the plain
+rotation and softmax in float32: ragged contexts on the edges of tiles, pages and ranges, one to sixteen query heads per
+kv head, and a step padded to the size of its graph."""
+
+import types
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from paged_llm_b200.kernels.ops import CudaOps
+    ops = CudaOps("cuda")
+    ops.set_compute_dtype(torch.bfloat16)
+    return ops
+
+
+def rotated(x, table):
+    """x [..., d] bfloat16 rotated by (cos, sin) [d / 2, 2] in float32, rounded back as the kernels store it."""
+    d = x.shape[-1]
+    a, b = x[..., :d // 2].float(), x[..., d // 2:].float()
+    c, s = table[:, 0], table[:, 1]
+    return torch.cat([a * c - b * s, b * c + a * s], -1).to(torch.bfloat16)
+
+
+EDGES = [1, 2, 15, 16, 17, 31, 32, 33, 127, 128, 129, 144, 513, 1000, 2049, 3500]
+
+
+@pytest.mark.parametrize("nh,nkv,d,ps,S,pad", [(32, 4, 64, 16, 40, 48), (32, 8, 64, 32, 24, 32), (32, 8, 128, 16, 21, 24),
+                                               (32, 2, 64, 48, 80, 96), (8, 8, 128, 64, 19, 19), (16, 1, 64, 16, 150, 192)])
+def test_even_ranges_against_plain_attention(ops, nh, nkv, d, ps, S, pad):
+    from paged_llm_b200.engine.context import AttentionPlan, HostBatch
+    G, W = nh // nkv, (nh + 2 * nkv) * d
+    k_lens = [EDGES[(i * 5) % len(EDGES)] for i in range(S)]
+    g = torch.Generator(device="cuda").manual_seed(S)
+    pages = [-(-n // ps) for n in k_lens]
+    order = torch.randperm(sum(pages) + 3, generator=torch.Generator().manual_seed(1)).int()
+    bt = torch.full((pad, max(pages) + 1), 10 ** 6, dtype=torch.int32)
+    kv = torch.full((sum(pages) + 3, 2, nkv, ps, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    qkv = torch.randn(pad, W, device="cuda", generator=g).to(torch.bfloat16)
+    table = torch.randn(4096, d // 2, 2, device="cuda", generator=g)
+    old, o = [], 0
+    for s, n in enumerate(k_lens):                        # all keys but the step's own are in the cache, the rest is NaN
+        mine = order[o:o + pages[s]]
+        bt[s, :pages[s]] = mine
+        o += pages[s]
+        both = torch.randn(2, n - 1, nkv, d, device="cuda", generator=g).to(torch.bfloat16)
+        flat = torch.full((2, pages[s] * ps, nkv, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        flat[:, :n - 1] = both
+        kv[mine.long().cuda()] = flat.view(2, pages[s], ps, nkv, d).permute(1, 0, 3, 2, 4)
+        old.append(both)
+    plan = ops.plan_attention([1] * S, k_lens, G, nkv, None, d, pad_requests=pad, fixed_capacity=True)
+    assert plan["even"] and plan["small"].reshape(-1, 4)[:, 3].max() > 1, "some request is meant to be split"
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.int32)).cuda()
+    small = plan["small"].reshape(-1, 4)
+    ap = AttentionPlan(dev(small), None, dev(plan["splits"]), len(small), 0, plan["max_splits"], plan["num_small_tokens"],
+                       plan["long_context"], plan["even"])
+    host = HostBatch([1] * S, [n - 1 for n in k_lens], [-1] * S)
+    ctx = types.SimpleNamespace(num_tokens=pad, num_seqs=pad, host=host, cu_seqlens_q=dev(list(range(S + 1)) + [S] * (pad - S)),
+                                seq_lens_k=dev(k_lens + [0] * (pad - S)), attention_plans={(G, nkv, None, d): ap}, padded=pad > S)
+    rope = types.SimpleNamespace(table=table, rotary_dim=d)
+    for _ in range(2):                                    # the second time finds the counters as the first left them
+        out = ops.paged_attention(qkv, nh, nkv, d, kv, bt.cuda(), ctx, d ** -0.5, None, rope=rope).float()
+    assert (out[S:] == 0).all()
+    for s, n in enumerate(k_lens):
+        q, k, v = (t.view(-1, d) for t in qkv[s].split([nh * d, nkv * d, nkv * d]))
+        q, k = rotated(q, table[n - 1]), rotated(k, table[n - 1])
+        slot = kv[bt[s, (n - 1) // ps], :, :, (n - 1) % ps]
+        # (the kernel may round one product of a rotated pair less than torch does: a neighbouring bfloat16)
+        torch.testing.assert_close(slot[0].float(), k.float(), atol=2 ** -20, rtol=2 ** -7, msg=f"request {s}: the cached key")
+        assert torch.equal(slot[1], v), f"request {s}: the cached value"
+        keys, vals = torch.cat([old[s][0], slot[0][None]]).float(), torch.cat([old[s][1], v[None]]).float()
+        score = torch.einsum("jgd,njd->jgn", q.float().view(nkv, G, d), keys) * d ** -0.5
+        want = torch.einsum("jgn,njd->jgd", score.softmax(-1), vals).reshape(-1)
+        # probabilities and the result are rounded to bfloat16 (2^-9 each), relative to values of up to 4.5
+        torch.testing.assert_close(out[s], want, atol=2 * 4.5 * 2 ** -9, rtol=2 ** -8, msg=f"request {s} of {n} keys")
+    assert ops.kernel_timeouts() == 0

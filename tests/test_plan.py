@@ -72,3 +72,39 @@ def test_long_context_decode_steps_are_split_further():
     assert is_long_context(8, 4, 148, 32, 8, 600, 3001) and not is_long_context(8, 4, 148, 32, 8, 600, 3000)
     # 64 requests x 4 kv heads: one block each either way, so there is no second class (and no second graph)
     assert not is_long_context(64, 4, 148, 32, 8, 600, 100000)
+
+
+@pytest.mark.parametrize("k_lens,nkv,pad", [([641] * 64, 4, 64), (list(range(131, 3501, 130)), 8, 32), ([1] * 40, 4, 48),
+                                             ([1, 4000] * 20, 8, 48), (list(range(70, 778, 5)), 4, 192), ([3000] * 16, 8, 16),
+                                             ([17] * 255 + [4000], 1, 256)])
+def test_even_ranges_cover_every_key_and_fit_the_graph(k_lens, nkv, pad):
+    """Steps that are cut into even ranges: every request has all its ranges, the list fits the capacity that a captured
+    graph has, whatever the lengths, and its shape does not depend on them; a range is never shorter than an even share of
+    128 keys, so no block starts for a handful."""
+    kw = dict(cluster_max=8, long_keys=600, slots=296)
+    S = len(k_lens)
+    plan = general([1] * S, k_lens, 8, nkv, None, pad_requests=pad, fixed_capacity=True, **kw)
+    assert plan["even"]
+    small, splits = plan["small"].reshape(-1, 4), plan["splits"].reshape(-1, 2)
+    real = small[small[:, 0] >= 0]
+    assert (small[len(real):] == -1).all() and len(small) == pad + 296 // nkv
+    for s, n in enumerate(k_lens):
+        mine = real[real[:, 0] == s]
+        assert sorted(mine[:, 2].tolist()) == list(range(splits[s, 0])) and (mine[:, 3] == splits[s, 0]).all()
+        assert splits[s, 0] <= min(plan["max_splits"], max(1, -(-n // 128)))
+    same = general([1] * S, [5] * (S - 1) + [max(k_lens)], 8, nkv, None, pad_requests=pad, fixed_capacity=True, **kw)
+    assert same["small"].size == plan["small"].size and same["max_splits"] == plan["max_splits"]
+    ends = [-(-k_lens[int(s)] // int(m)) for s, _, _, m in real]
+    assert ends[0] <= max(max(k_lens), 128) and (len(set(k_lens)) > 1 or len(set(ends)) == 1)
+
+
+def test_even_ranges_beside_prompt_portions():
+    """A step of mixed items that replays a graph: the same capacity with and without decoding requests."""
+    kw = dict(cluster_max=8, long_keys=600, slots=296, pad_requests=64, fixed_capacity=True, pad_tokens=448)
+    busy = general([1] * 33 + [200, 100], [128 + 40 * i for i in range(33)] + [1200, 1100], 4, 8, None, **kw)
+    alone = general([400], [400], 4, 8, None, **kw)
+    for key in ("small", "large", "splits"):
+        assert busy[key].size == alone[key].size
+    assert busy["max_splits"] == alone["max_splits"] and busy["num_small_tokens"] == alone["num_small_tokens"]
+    small = busy["small"].reshape(-1, 4)
+    assert set(small[small[:, 0] >= 0][:, 0].tolist()) == set(range(33)) and (alone["small"] == -1).all()
