@@ -30,10 +30,12 @@ _DTYPE_CODE = {torch.float32: PL_F32, torch.bfloat16: PL_BF16}
 class LazyNorm:
     """RMSNorm(x) * weight that no kernel has formed yet: the product that comes next
     normalises while it loads.  `part` holds the sums of squares of x that the product
-    in front left (per 16 columns and token)."""
+    in front left (per 16 columns and token).  `scaled` (steps of 17 tokens and more): x * weight
+    as bfloat16, for a product that multiplies by 1 / rms(x) afterwards; `part` then is per 128
+    columns."""
 
-    def __init__(self, x: torch.Tensor, part: torch.Tensor, weight: torch.Tensor, eps: float):
-        self.x, self.part, self.weight, self.eps = x, part, weight, eps
+    def __init__(self, x: torch.Tensor, part: torch.Tensor, weight: torch.Tensor, eps: float, scaled: torch.Tensor | None = None):
+        self.x, self.part, self.weight, self.eps, self.scaled = x, part, weight, eps, scaled
         self.shape = x.shape
         self.dtype = torch.bfloat16
 
@@ -84,7 +86,7 @@ def load_module(name: str) -> ctypes.CDLL:
 
 # Every wait inside a kernel (on an mbarrier of a TMA ring or of tcgen05) is bounded; a wait that
 # gives up adds one to a counter of its module, which these exports read.
-_TIMEOUT_EXPORTS = ("pl_gemm_skinny_timeouts", "pl_gemm_tc_timeouts", "pl_attention_tc_timeouts")
+_TIMEOUT_EXPORTS = ("pl_gemm_skinny_timeouts", "pl_gemm_mid_timeouts", "pl_gemm_tc_timeouts", "pl_attention_tc_timeouts")
 
 
 def _check(lib, rc: int) -> None:
@@ -124,6 +126,8 @@ class CudaOps:
         self._attn_fn = None
         self.launches = 0                 # kernels of this package launched so far
         self.use_skinny = True            # few-token products on this package's weight-streaming kernel
+        # from 17 tokens to this many, products on the tcgen05 kernel that splits k over clusters (0: none)
+        self.mid_tokens = 0 if os.environ.get("PAGED_LLM_B200_NO_GEMM_MID") else self.core.pl_gemm_mid_max_tokens()
         # Many tokens: this package's tcgen05 kernel (pairs of blocks on 256 x 256 tiles, fused epilogues) where it is at least
         # as fast as the library product followed by the elementwise kernel.  Measured: the gate/up product
         # with SiLU-mul from 2,048 tokens on (77 us against 87 us, timed alone); the narrower products and fewer
@@ -453,6 +457,23 @@ class CudaOps:
         M, K = h.shape
         return self.use_skinny and h.dtype == torch.bfloat16 and 1 <= M <= 16 and K >= 32 and K % 32 == 0
 
+    def _mid_ok(self, h, w: torch.Tensor, align: int, width: int) -> bool:
+        """A middling number of tokens (see gemm_mid.cu); the outputs' width a multiple of `align`.  `width`: the model's.  At
+        Llama-3-8B's 4,096 the gate and up products alone are 235 MB, the launches between products weigh little and the
+        library's wider tiles read W faster: 4,115 against 4,192 us for a prompt of 61 tokens; at 2,048 the whole step
+        gains 3 to 22 % (20 requests 1,133 -> 886 us, 48 requests of Llama-3.2-1B 1,147 -> 1,020, its prompt of 40
+        tokens 1,212 -> 1,172)."""
+        M, K = h.shape
+        return (16 < M <= self.mid_tokens and width < 4096 and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+                and K % 64 == 0 and w.shape[0] % align == 0 and w.is_contiguous()
+                and ((h.scaled is not None and K % 128 == 0) if isinstance(h, LazyNorm) else h.is_contiguous()))
+
+    def _mid_args(self, h):
+        """(X, its row stride, partial sums, eps) for a product of `gemm_mid.cu`."""
+        if isinstance(h, LazyNorm):
+            return self._p(h.scaled), h.shape[1], self._p(h.part), c_float(h.eps)
+        return self._p(h), h.shape[1], c_void_p(0), c_float(0.0)
+
     def _gemm_tc_ok(self, h, w: torch.Tensor, kind: str) -> bool:
         M, K = h.shape
         return (kind in self.gemm_tc_for and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
@@ -476,6 +497,13 @@ class CudaOps:
         assert w.shape[1] == K and w.is_contiguous()
         if self._skinny_ok(h, N) and w.dtype == torch.bfloat16:
             return self._skinny_linear(h, w, out_float32)
+        if self._mid_ok(h, w, 4, K):
+            x, ldx, part, eps = self._mid_args(h)
+            out = torch.empty((M, N), dtype=torch.float32 if out_float32 else torch.bfloat16, device=self.device)
+            _check(self.core, self.core.pl_gemm_mid(x, ldx, self._p(w), self._p(out), N, M, N, K, 1 if out_float32 else 0,
+                                                    part, eps, self._stream))
+            self.launches += 1
+            return out
         h = self.materialize(h)
         assert h.is_contiguous()
         if self._gemm_tc_ok(h, w, "plain") and N % 8 == 0:
@@ -510,11 +538,20 @@ class CudaOps:
         forms while loading; else the product is followed by the fused sum+norm kernel."""
         M, K = h.shape
         N = w.shape[0]
-        if not isinstance(h, LazyNorm) and self._skinny_ok(h, N) and N % 16 == 0 and N % 32 == 0:
+        few = self._skinny_ok(h, N) and N % 16 == 0 and N % 32 == 0
+        mid = not out_float32 and self._mid_ok(h, w, 128, N) and norm_w.is_contiguous()
+        if not isinstance(h, LazyNorm) and (few or mid):
             assert x.dtype == torch.float32 and x.is_contiguous() and x.shape == (M, N) and h.is_contiguous()
-            if self._norm_part is None or self._norm_part.numel() < N:
+            if self._norm_part is None or self._norm_part.numel() < 2 * N:
                 self._norm_part_keep.append(self._norm_part)        # captured graphs hold the old address
-                self._norm_part = torch.zeros(max(N, 1 << 16), dtype=torch.float32, device=self.device)
+                self._norm_part = torch.zeros(max(2 * N, 1 << 16), dtype=torch.float32, device=self.device)
+        if not isinstance(h, LazyNorm) and mid:
+            scaled = torch.empty((M, N), dtype=torch.bfloat16, device=self.device)
+            _check(self.core, self.core.pl_gemm_mid_add(self._p(h), K, self._p(w), self._p(x), self._p(scaled), self._p(norm_w),
+                                                        self._code(norm_w), M, N, K, self._p(self._norm_part), self._stream))
+            self.launches += 1
+            return LazyNorm(x, self._norm_part, norm_w, eps, scaled)
+        if not isinstance(h, LazyNorm) and few:
             _check(self.core, self.core.pl_gemm_skinny_add(self._p(h), K, self._p(w), self._p(x), M, N, K,
                                                            self._p(self._norm_part), self._stream))
             self.launches += 1
@@ -538,6 +575,13 @@ class CudaOps:
             out = torch.empty((M, I), dtype=torch.bfloat16, device=self.device)
             _check(self.core, self.core.pl_gemm_skinny_silu(x, ldx, self._p(w_gate_up), self._p(out), I, M, I, K,
                                                             part, nw, nwc, eps, ACTIVATIONS[activation], self._stream))
+            self.launches += 1
+            return out
+        if self._mid_ok(h, w_gate_up, 4, K):
+            x, ldx, part, eps = self._mid_args(h)
+            out = torch.empty((M, I), dtype=torch.bfloat16, device=self.device)
+            _check(self.core, self.core.pl_gemm_mid_silu(x, ldx, self._p(w_gate_up), self._p(out), I, M, I, K,
+                                                         ACTIVATIONS[activation], part, eps, self._stream))
             self.launches += 1
             return out
         h = self.materialize(h)
@@ -1337,8 +1381,8 @@ class CudaOps:
         if T > real or getattr(ctx, "padded", False):
             # Rows that pad the step to the size of its graph.  The split-context kernels zero them themselves
             # (a fill kernel between two kernels of a layer would keep them from overlapping: 0.97 against 0.92 ms
-            # per step at 12 requests); a step with large items too is not padded in practice and gets the fill.
-            if plan.n_large:
+            # per step at 12 requests).
+            if not plan.n_small:
                 out.zero_()
             else:
                 p.pad_seqs, p.pad_to = ctx.num_seqs, T
@@ -1403,7 +1447,7 @@ class CudaOps:
                 _check(self.core, self.core.pl_attention_combine(ctypes.byref(p), self._code(out), self._stream))
                 self.launches += 1
         if plan.n_large:
-            p.scratch, p.scratch_floats = 0, 0
+            p.scratch, p.scratch_floats, p.pad_to = 0, 0, 0
             p.work, p.n_work, p.is_small = plan.large.data_ptr(), plan.n_large, 0
             p.max_splits = 1
             _check(lib, fn(ctypes.byref(p), self._stream))
