@@ -9,7 +9,10 @@
 // row (counts for top-k, probability mass for top-p) and a suffix sum over its 256
 // bins; tokens that tie with a threshold all stay.  Mass is summed in fixed point
 // (2^-40 units in 64-bit integers), so the sums do not depend on the order in
-// which threads arrive.  The draw is argmax(logit/T + g), g = -log(-log u), which
+// which threads arrive.  A row is read three times: for its largest and smallest logit; for its mass and a
+// histogram of the distances from the largest; and to gather what can pass the filters, in most rows a few
+// hundred tokens, which the radix search and the draw then go over in shared memory (a row whose
+// candidates do not fit is searched in place).  The draw is argmax(logit/T + g), g = -log(-log u), which
 // samples the softmax of the kept tokens; u comes from a counter-based stream
 // u(seed, counter, token index) (splitmix64), so a request's draw does not
 // depend on the rest of the batch.
@@ -160,9 +163,15 @@ struct SampleShared {
     unsigned int cnt[256], piece[3][256];      // this block's histogram of the digit at hand
     unsigned int key_lo, key_hi;               // smallest and largest key of its part of the row
     unsigned long long z;                      // mass of its part of the row
+    unsigned long long list_z;                 // mass of the candidates it gathered
     float best_v;                              // its best candidate of the draw
     int best_i;
 };
+
+// Candidates of a row that are gathered at most, and the width of a bin of the histogram that finds them, in units of
+// logit / T: 256 bins reach 32 below the largest.
+constexpr int LIST = 2048;
+constexpr float BINS_PER_UNIT = 8.f;
 
 // One row per block (CL == 1), or per thread-block cluster of CL blocks that take a part of the row each (large
 // vocabularies: a block alone needs seven sweeps over half a megabyte).  Every block of a cluster adds up the
@@ -225,13 +234,28 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
     uint32_t key_floor = 0;                                   // tokens with ordered_key >= key_floor stay
 
     const bool use_k = top_k > 0 && top_k < V, use_p = top_p < 1.0f;
+    __shared__ float list_x[LIST];                            // this block's candidates: logit / T and token
+    __shared__ int list_i[LIST];
+    __shared__ unsigned int list_n;
+    bool listed = false;                                      // the candidates hold all tokens that stay
+    // f(i, logit / T) for the tokens that may stay
+    auto for_each_candidate = [&](auto f) {
+        if (listed) {
+            for (unsigned e = tid; e < list_n; e += blockDim.x) f(list_i[e], list_x[e]);
+        } else {
+            for_each_logit(row, lo, hi, vec, [&](int i, float v) { f(i, v * inv_t); });
+        }
+    };
     if (use_k || use_p) {
         __shared__ unsigned int cnt_all[256], warp_cnt[8];
         __shared__ unsigned long long mass[256], warp_mass[8];
         __shared__ unsigned int pick_k, pick_p, need_k;
         __shared__ unsigned long long above_p, limit_p;
+        __shared__ unsigned int coarse_cut;
+        if (tid < 256) sh.cnt[tid] = 0u;
         if (tid == 0) {
-            sh.z = 0ull;
+            sh.z = sh.list_z = 0ull;
+            list_n = 0u;
             need_k = (unsigned)top_k;
             above_p = 0ull;
             sh.key_lo = 0xFFFFFFFFu;
@@ -274,17 +298,85 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
         // value each (shared memory adds 32-bit integers natively, 64-bit ones by compare-and-swap: 3.4 times
         // slower here); each stays below 2^32 for up to 2^21 tokens.
         auto fixed_mass = [&](float x) { return __float2ull_rn(expf(x - mx) * 8589934592.0f); };
-        if (use_p) {
+        // The row's mass, and how many tokens lie how far below the largest (monotone in the logit, so that a bin and all
+        // above it are the largest tokens; what is further off, or not a number, is not counted: bin 0).
+        auto coarse = [&](float x) {
+            const float far = (mx - x) * BINS_PER_UNIT;
+            return far < 255.f ? 255 - (int)far : 0;
+        };
+        {
             unsigned long long z = 0ull;
-            for_each_logit(row, lo, hi, vec, [&](int, float v) { z += fixed_mass(v * inv_t); });
+            for_each_logit(row, lo, hi, vec, [&](int, float v) {
+                const float x = v * inv_t;
+                if (use_p) z += fixed_mass(x);
+                const int bin = coarse(x);
+                if (bin > 0) atomicAdd(&sh.cnt[bin], 1u);
+            });
+            if (use_p) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-            if ((tid & 31) == 0) atomicAdd(&sh.z, z);
+                for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+                if ((tid & 31) == 0) atomicAdd(&sh.z, z);
+            }
             sync_row();
-            if (tid == 0) {
+            if (tid == 0 && use_p) {
                 unsigned long long total = 0ull;
                 for (int k = 0; k < CL; ++k) total += peer(k)->z;
                 limit_p = (unsigned long long)((double)top_p * (double)total);
+            }
+            if (tid < 32) {
+                // the bin to gather from: with top-k the highest that has k tokens in it and above, else the lowest whose
+                // tokens and all above fit the list; 0: none.  Lane l holds bins 8 l .. 8 l + 7.
+                unsigned int in[8], sum = 0u;
+#pragma unroll
+                for (int j = 7; j >= 0; --j) {
+                    unsigned int c = 0u;
+                    for (int k = 0; k < CL; ++k) c += peer(k)->cnt[8 * tid + j];
+                    sum += c;
+                    in[j] = sum;
+                }
+                unsigned int above = sum;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const unsigned int c = __shfl_down_sync(0xffffffffu, above, off);
+                    if (tid + off < 32) above += c;
+                }
+                above -= sum;                                 // tokens in the bins of the lanes behind
+                int best = use_k ? -1 : 256;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const unsigned int n = above + in[j];
+                    if (use_k && n >= (unsigned)top_k && n <= (unsigned)LIST) best = 8 * tid + j;
+                    if (!use_k && n <= (unsigned)LIST) best = min(best, 8 * tid + j);
+                }
+                best = use_k ? __reduce_max_sync(0xffffffffu, best) : __reduce_min_sync(0xffffffffu, best);
+                if (tid == 0) coarse_cut = best >= 0 && best < 256 ? (unsigned)max(best, 1) : 0u;
+            }
+            __syncthreads();
+        }
+        const int cut = (int)coarse_cut;                      // the same in all blocks of the row
+        if (cut > 0) {
+            unsigned long long z = 0ull;
+            for_each_logit(row, lo, hi, vec, [&](int i, float v) {
+                const float x = v * inv_t;
+                if (coarse(x) < cut) return;
+                const unsigned at = atomicAdd(&list_n, 1u);   // (at most LIST in the whole row)
+                list_x[at] = x;
+                list_i[at] = i;
+                if (use_p) z += fixed_mass(x);
+            });
+            if (use_p && !use_k) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+                if ((tid & 31) == 0) atomicAdd(&sh.list_z, z);
+            }
+            sync_row();
+            // With k tokens or more in the list the k-th is among them, and whatever top-p would let in beyond it falls to
+            // top-k.  With top-p alone the list must hold more mass than is allowed above the threshold.
+            listed = use_k;
+            if (!use_k) {
+                unsigned long long held = 0ull;
+                for (int k = 0; k < CL; ++k) held += peer(k)->list_z;
+                listed = held > limit_p;
             }
         }
         uint32_t prefix_k = 0, prefix_p = 0;                  // the digits found so far, most significant first
@@ -296,8 +388,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
                 sh.piece[0][tid] = sh.piece[1][tid] = sh.piece[2][tid] = 0u;
             }
             __syncthreads();
-            for_each_logit(row, lo, hi, vec, [&](int, float v) {
-                const float x = v * inv_t;
+            for_each_candidate([&](int, float x) {
                 const uint32_t key = spread(ordered_key(x));
                 const uint32_t high = digit == digits - 1 ? 0u : key >> (shift + 8);
                 const uint32_t bin = (key >> shift) & 255u;
@@ -389,8 +480,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
     }
     const uint64_t seed = seeds[r], counter = counters[r];
     MaxIdx best{-INFINITY, 0x7fffffff};
-    for_each_logit(row, lo, hi, vec, [&](int i, float v) {
-        const float x = v * inv_t;
+    for_each_candidate([&](int i, float x) {
         if (ordered_key(x) < key_floor) return;
         const float u = uniform01(seed, counter, (uint64_t)i);
         const float score = x - logf(-logf(u));

@@ -845,3 +845,32 @@ def test_window_edge_is_exact(ops, dtype, d):
         qs[L - nq:] = q.float()
         full = plain_llama.causal_attention(qs, keys[0], vals[0], d ** -0.5, window=window)[L - nq:].reshape(nq, nh * d)
         torch.testing.assert_close(out, full, atol=2e-2, rtol=2e-2, msg=f"nq={nq}")
+
+
+@pytest.mark.parametrize("kind", ["flat", "peaked", "ties", "masked", "infinite"])
+@pytest.mark.parametrize("top_k,top_p", [(50, 0.9), (0, 0.9), (3000, 1.0), (1, 1.0), (50, 1.0), (0, 0.999)])
+def test_sampling_from_gathered_candidates_keeps_the_same_tokens(ops, kind, top_k, top_p):
+    """Rows whose candidates fit the list, rows whose do not (flat ones), ties across the bins of the histogram, masked
+    tokens and infinities: no token outside the reference's filter is ever drawn."""
+    rows, V = 64, 40000
+    row = randn(V, seed=3, std={"flat": 1e-4, "peaked": 6.0}.get(kind, 2.0))
+    if kind == "ties":
+        row = (row * 2).round() / 2
+    if kind == "masked":
+        row[1000:] = -math.inf
+    if kind == "infinite":
+        row[7] = math.inf
+    logits = row.expand(rows, V).contiguous()
+    got = ops.sample(logits, np.full(rows, 0.7, np.float32), np.full(rows, top_k, np.int32), np.full(rows, top_p, np.float32),
+                     np.arange(rows, dtype=np.uint64), np.full(rows, 5, np.uint64)).long()
+    assert ((got >= 0) & (got < V)).all()
+    if kind == "infinite":
+        return
+    x = (row * np.float32(1 / np.float32(0.7))).double()
+    p = torch.softmax(x, 0)
+    order = x.sort(descending=True)
+    above = torch.searchsorted(-order.values, -x, right=False)                   # how many tokens are larger
+    mass = torch.cat([torch.zeros(1, dtype=torch.float64, device="cuda"), p[order.indices].cumsum(0)])[above]
+    # (masses are float32 exponentials in parts of 2^-33 of the largest: a token within 1e-5 of the limit may go either way)
+    keep = (mass <= top_p + 1e-5) & ((above < top_k) if 0 < top_k < V else torch.ones_like(mass, dtype=torch.bool))
+    assert keep[got].all()
