@@ -490,8 +490,8 @@ class CudaOps:
 
     def linear(self, h, w: torch.Tensor, out_float32: bool = False) -> torch.Tensor:
         """h [M, K] @ w[N, K]^T.  float32: this package's CUDA-core kernel; bfloat16 with few
-        tokens: this package's weight-streaming kernel; else the library product with
-        float32 accumulation.  `h` may be a `LazyNorm`."""
+        tokens: this package's weight-streaming kernel, with up to 64 its tcgen05 kernel that splits k
+        (see `_mid_ok`); else the library product with float32 accumulation.  `h` may be a `LazyNorm`."""
         M, K = h.shape
         N = w.shape[0]
         assert w.shape[1] == K and w.is_contiguous()
@@ -535,7 +535,7 @@ class CudaOps:
     def linear_add_rms_norm(self, h, w, x, norm_w, eps, out_float32: bool = False):
         """x += h @ w^T (float32 stream, in place), then RMSNorm(x) * norm_w.  With few tokens
         the product's epilogue adds and the result is a `LazyNorm` that the next product
-        forms while loading; else the product is followed by the fused sum+norm kernel."""
+        forms while loading, with up to 64 one that the next product divides after summing; else the product is followed by the fused sum+norm kernel."""
         M, K = h.shape
         N = w.shape[0]
         few = self._skinny_ok(h, N) and N % 16 == 0 and N % 32 == 0
@@ -1341,9 +1341,9 @@ class CudaOps:
                       softcap=None, slopes=None, chunk=None, value_from_key=False) -> torch.Tensor:
         """The mixer's whole front: fused q/k/v projection, rotary positions on q and k, k and v written
         to the cache, attention over the pages.  Returns [T, nh * d].  It is `qkv_rope_write` followed by
-        `paged_attention`, but for a decode step of more than 16 tokens (the projection is a library
-        product then, without an epilogue) rotation and cache write happen inside the attention
-        kernel instead of in a kernel of their own."""
+        `paged_attention`, but for a decode step of more than 16 tokens (the projection's epilogue does
+        not rotate then) rotation and cache write happen inside the attention kernel instead of in
+        a kernel of their own."""
         M = h.shape[0]
         plan = ctx.attention_plans.get(attention_plan_key(nh, nkv, window, d, chunk))
         inside = (plan is not None and write and softcap is None and slopes is None and position is not None
