@@ -164,6 +164,7 @@ struct SampleShared {
     unsigned int key_lo, key_hi;               // smallest and largest key of its part of the row
     unsigned long long z;                      // mass of its part of the row
     unsigned long long list_z;                 // mass of the candidates it gathered
+    unsigned int list_n;                       // and their number
     float best_v;                              // its best candidate of the draw
     int best_i;
 };
@@ -236,14 +237,17 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
     const bool use_k = top_k > 0 && top_k < V, use_p = top_p < 1.0f;
     __shared__ float list_x[LIST];                            // this block's candidates: logit / T and token
     __shared__ int list_i[LIST];
-    __shared__ unsigned int list_n;
     bool listed = false;                                      // the candidates hold all tokens that stay
+    // logit / T: the same rounded value in every sweep.  (A product that the compiler fuses with the subtraction behind it
+    // in one sweep and not in another puts a token on the edge of a bin into the one here and into the other there, and
+    // tokens whose rounded values tie into different bins.)
+    auto scaled = [&](float v) { return __fmul_rn(v, inv_t); };
     // f(i, logit / T) for the tokens that may stay
     auto for_each_candidate = [&](auto f) {
         if (listed) {
-            for (unsigned e = tid; e < list_n; e += blockDim.x) f(list_i[e], list_x[e]);
+            for (unsigned e = tid; e < sh.list_n; e += blockDim.x) f(list_i[e], list_x[e]);
         } else {
-            for_each_logit(row, lo, hi, vec, [&](int i, float v) { f(i, v * inv_t); });
+            for_each_logit(row, lo, hi, vec, [&](int i, float v) { f(i, scaled(v)); });
         }
     };
     if (use_k || use_p) {
@@ -255,7 +259,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
         if (tid < 256) sh.cnt[tid] = 0u;
         if (tid == 0) {
             sh.z = sh.list_z = 0ull;
-            list_n = 0u;
+            sh.list_n = 0u;
             need_k = (unsigned)top_k;
             above_p = 0ull;
             sh.key_lo = 0xFFFFFFFFu;
@@ -265,7 +269,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
         {
             uint32_t klo = 0xFFFFFFFFu, khi = 0u;
             for_each_logit(row, lo, hi, vec, [&](int, float v) {
-                const uint32_t key = ordered_key(v * inv_t);
+                const uint32_t key = ordered_key(scaled(v));
                 klo = min(klo, key);
                 khi = max(khi, key);
             });
@@ -307,7 +311,7 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
         {
             unsigned long long z = 0ull;
             for_each_logit(row, lo, hi, vec, [&](int, float v) {
-                const float x = v * inv_t;
+                const float x = scaled(v);
                 if (use_p) z += fixed_mass(x);
                 const int bin = coarse(x);
                 if (bin > 0) atomicAdd(&sh.cnt[bin], 1u);
@@ -357,11 +361,13 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
         if (cut > 0) {
             unsigned long long z = 0ull;
             for_each_logit(row, lo, hi, vec, [&](int i, float v) {
-                const float x = v * inv_t;
+                const float x = scaled(v);
                 if (coarse(x) < cut) return;
-                const unsigned at = atomicAdd(&list_n, 1u);   // (at most LIST in the whole row)
-                list_x[at] = x;
-                list_i[at] = i;
+                const unsigned at = atomicAdd(&sh.list_n, 1u);
+                if (at < (unsigned)LIST) {                    // (at most LIST in the whole row, by the histogram)
+                    list_x[at] = x;
+                    list_i[at] = i;
+                }
                 if (use_p) z += fixed_mass(x);
             });
             if (use_p && !use_k) {
@@ -372,12 +378,13 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
             sync_row();
             // With k tokens or more in the list the k-th is among them, and whatever top-p would let in beyond it falls to
             // top-k.  With top-p alone the list must hold more mass than is allowed above the threshold.
-            listed = use_k;
-            if (!use_k) {
-                unsigned long long held = 0ull;
-                for (int k = 0; k < CL; ++k) held += peer(k)->list_z;
-                listed = held > limit_p;
+            listed = true;
+            unsigned long long held = 0ull;
+            for (int k = 0; k < CL; ++k) {
+                held += peer(k)->list_z;
+                listed = listed && peer(k)->list_n <= (unsigned)LIST;
             }
+            if (!use_k) listed = listed && held > limit_p;
         }
         uint32_t prefix_k = 0, prefix_p = 0;                  // the digits found so far, most significant first
         for (int digit = digits - 1; digit >= 0; --digit) {
