@@ -128,6 +128,9 @@ class CudaOps:
         self.use_skinny = True            # few-token products on this package's weight-streaming kernel
         # from 17 tokens to this many, products on the tcgen05 kernel that splits k over clusters (0: none)
         self.mid_tokens = 0 if os.environ.get("PAGED_LLM_B200_NO_GEMM_MID") else self.core.pl_gemm_mid_max_tokens()
+        # ... in models of these widths, `mid_width_per_token` wide per token at least, and for heads of up to so many features:
+        # as many as there are rows for blocks at a time (see `_mid_ok` and `linear`)
+        self.mid_widths, self.mid_width_per_token, self.mid_features = (640, 4096), 20, 2 * self.num_sms * 128
         # Many tokens: this package's tcgen05 kernel (pairs of blocks on 256 x 256 tiles, fused epilogues) where it is at least
         # as fast as the library product followed by the elementwise kernel.  Measured: the gate/up product
         # with SiLU-mul from 2,048 tokens on (77 us against 87 us, timed alone); the narrower products and fewer
@@ -458,13 +461,27 @@ class CudaOps:
         return self.use_skinny and h.dtype == torch.bfloat16 and 1 <= M <= 16 and K >= 32 and K % 32 == 0
 
     def _mid_ok(self, h, w: torch.Tensor, align: int, width: int) -> bool:
-        """A middling number of tokens (see gemm_mid.cu); the outputs' width a multiple of `align`.  `width`: the model's.  At
-        Llama-3-8B's 4,096 the gate and up products alone are 235 MB, the launches between products weigh little and the
-        library's wider tiles read W faster: 4,115 against 4,192 us for a prompt of 61 tokens; at 2,048 the whole step
-        gains 3 to 22 % (20 requests 1,133 -> 886 us, 48 requests of Llama-3.2-1B 1,147 -> 1,020, its prompt of 40
-        tokens 1,212 -> 1,172)."""
+        """A middling number of tokens (see gemm_mid.cu); the outputs' width a multiple of `align`.  `width`: the model's.
+
+        In models of width 4,096 on the library's wider tiles read W faster where it is large: gate and up of 14,336 features
+        44.4 against 45.7 us at 24 tokens, and a prompt of 61 tokens 4,115 against 4,192 us (o and down are ahead here,
+        10.6 against 12.6 and 25.7 against 28.4: a rule by product is not made).  At 2,048 a whole step gains 3 to 25 %
+        (20 requests 1,133 -> 886 us, 48 requests of Llama-3.2-1B 1,147 -> 1,020, its prompt of 40 tokens 1,212 -> 1,172).
+        In narrow models W is small, every block's read of all of X weighs more, and the more so the more tokens.  The four
+        products of a layer (q/k/v of 1.5 widths, gate and up of 2.75), library and here, us:
+
+            width    17 tokens      33 tokens      64 tokens
+              512   18.8  18.1     19.1  20.7     18.9  23.4
+              768   22.9  19.7     24.5  21.4     22.5  23.7
+            1,024   25.9  21.3     25.4  23.1     25.0  26.2
+            1,280   28.6  23.8     29.6  26.4     29.7  29.1
+            2,048   40.1  32.5     41.1  34.9     40.7  38.9
+            3,072   59.4  52.5     59.4  55.5     59.6  60.0
+
+        The line is a width of 20 per token, and of 640 (32 tokens there: 21.3 and 21.0)."""
         M, K = h.shape
-        return (16 < M <= self.mid_tokens and width < 4096 and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+        return (16 < M <= self.mid_tokens and self.mid_widths[0] <= width < self.mid_widths[1]
+                and M * self.mid_width_per_token <= width and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
                 and K % 64 == 0 and w.shape[0] % align == 0 and w.is_contiguous()
                 and ((h.scaled is not None and K % 128 == 0) if isinstance(h, LazyNorm) else h.is_contiguous()))
 
@@ -491,13 +508,15 @@ class CudaOps:
     def linear(self, h, w: torch.Tensor, out_float32: bool = False) -> torch.Tensor:
         """h [M, K] @ w[N, K]^T.  float32: this package's CUDA-core kernel; bfloat16 with few
         tokens: this package's weight-streaming kernel, with up to 64 its tcgen05 kernel that splits k
-        (see `_mid_ok`); else the library product with float32 accumulation.  `h` may be a `LazyNorm`."""
+        (see `_mid_ok`; a head of more features than its blocks have rows for at a time cannot split k, and the
+        library reads it faster: 128,256 features, K = 2,048, 83 against 93 us at 17 tokens and 98 against 107 at 64);
+        else the library product with float32 accumulation.  `h` may be a `LazyNorm`."""
         M, K = h.shape
         N = w.shape[0]
         assert w.shape[1] == K and w.is_contiguous()
         if self._skinny_ok(h, N) and w.dtype == torch.bfloat16:
             return self._skinny_linear(h, w, out_float32)
-        if self._mid_ok(h, w, 4, K):
+        if N <= self.mid_features and self._mid_ok(h, w, 4, K):
             x, ldx, part, eps = self._mid_args(h)
             out = torch.empty((M, N), dtype=torch.float32 if out_float32 else torch.bfloat16, device=self.device)
             _check(self.core, self.core.pl_gemm_mid(x, ldx, self._p(w), self._p(out), N, M, N, K, 1 if out_float32 else 0,
