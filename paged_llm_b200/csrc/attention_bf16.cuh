@@ -277,9 +277,10 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
     pdl_launch_dependents();
     // A block of a decode step waits for the kernel in front only after it has asked for its
     // first keys: lengths, lists, block tables and all keys but the step's own are older than the step.
+    const int padding = attn_padding_from(p);
     if (!EARLY) {
         pdl_wait();
-        attn_zero_padding<__nv_bfloat16>(p);
+        attn_zero_padding<__nv_bfloat16>(p, padding);
     }
     // kv heads of an item side by side: the list's longest-first order holds over heads
     const AttnItem it = CLUSTER ? attn_cluster_item(p, blockIdx.x / (p.cluster * p.nkv), blockIdx.x % p.cluster, p.cluster)
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
     if (!it.valid) {                 // the same for all blocks of a cluster
         if (EARLY) {
             pdl_wait();
-            attn_zero_padding<__nv_bfloat16>(p);
+            attn_zero_padding<__nv_bfloat16>(p, padding);
         }
         return;
     }
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
     }
     if (EARLY) {
         pdl_wait();
-        attn_zero_padding<__nv_bfloat16>(p);
+        attn_zero_padding<__nv_bfloat16>(p, padding);
         if (!ROPE) {                                      // (with ROPE they are made further down instead)
 #pragma unroll
             for (int t = 0; t < STAGES - 1; ++t)

@@ -64,9 +64,10 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(AttnParams p, cons
     // lengths, lists, block tables and all keys but the step's own are older than the step: they are read before the wait
     const AttnItem it = CLUSTER ? attn_cluster_item(p, blockIdx.x / (p.cluster * p.nkv), blockIdx.x % p.cluster, p.cluster)
                                 : attn_decode_item(p, blockIdx.x / p.nkv, 16, 32);
+    const int padding = attn_padding_from(p);
     if (!it.valid) {                                        // the same for all blocks of a cluster
         pdl_wait();
-        attn_zero_padding<__nv_bfloat16>(p);
+        attn_zero_padding<__nv_bfloat16>(p, padding);
         return;
     }
     unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)dec_smem + 1023) & ~(uintptr_t)1023);
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(AttnParams p, cons
         for (int k = 0; k < 4; ++k) angle[k] = __ldg(cs + k);
     }
     pdl_wait();
-    attn_zero_padding<__nv_bfloat16>(p);
+    attn_zero_padding<__nv_bfloat16>(p, padding);
     if (!ROPE) {
         asm volatile("fence.proxy.async;\n" ::: "memory");        // the kernel in front wrote them by ordinary stores
         for (; asked < min(STAGES, count); ++asked) ask(asked);

@@ -20,8 +20,9 @@ __device__ __forceinline__ void f32_copy(float* dst, const float* src, int bytes
 template <int NC>
 __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
     pdl_launch_dependents();
+    const int padding = attn_padding_from(p);
     pdl_wait();
-    attn_zero_padding<float>(p);
+    attn_zero_padding<float>(p, padding);
     const AttnItem it = attn_decode_item(p, blockIdx.x / p.nkv, F32_ROWS, F32_KEYS);
     if (!it.valid) return;
     extern __shared__ __align__(16) float smem[];
