@@ -67,13 +67,19 @@ def even_max_splits(scratch_rows: int, max_splits: int) -> int:
     return int(max(4, min(max_splits, 2048 // max(scratch_rows, 1))))
 
 
+# Contexts are rounded up to multiples of this many keys before they are cut: a plan then changes only when a context grows
+# past another multiple, which is when a replayed step makes its plan anew, and never depends on the step it was made for.
+GRAIN = 128
+
+
 def split_evenly(keys: np.ndarray, extra: int, max_splits: int) -> np.ndarray:
     """Ranges per request so that the blocks of a step end at about the same time although the requests' contexts differ
     (131 to 3,500 keys in one batch: a block per request and kv head walks 3,500 keys alone while most others have long
     ended).  `extra` ranges per kv head are resident at a time, and fit the lists beside one per request; of a few lengths
     of a range, none below an even share, the one after which the last block should end first."""
+    keys = -(-keys // GRAIN) * GRAIN
     total, longest = int(keys.sum()), int(keys.max())
-    share = max(128, -(-total // extra))
+    share = max(GRAIN, -(-total // extra))
     best = None
     for length in [longest] + [int(share * f) for f in (1.0, 1.15, 1.35, 1.6, 2.0, 2.7, 4.0)]:
         ns = np.clip(-(-keys // length), 1, max_splits)
@@ -85,6 +91,11 @@ def split_evenly(keys: np.ndarray, extra: int, max_splits: int) -> np.ndarray:
         if best is None or end < best[0]:
             best = (end, ns)
     return best[1].astype(np.int32)
+
+
+def longest_first(keys: np.ndarray, ns: np.ndarray) -> np.ndarray:
+    """Order of the requests of such a step in its list: by the length of their ranges."""
+    return np.argsort(-(-(-keys // GRAIN) * GRAIN // ns), kind="stable")
 
 
 def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_splits, fixed_capacity,
@@ -99,7 +110,7 @@ def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_sp
         lk = np.asarray(k_lens, np.int64)
         most = even_max_splits(n_req, max_splits)
         ns = split_evenly(lk, extra, most)
-        order = np.argsort(-(lk // ns), kind="stable").astype(np.int32)          # long ranges first
+        order = longest_first(lk, ns).astype(np.int32)
         many = ns[order]
         first = np.cumsum(many) - many
         total = int(ns.sum())
@@ -216,8 +227,8 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
             large.append((k_lens[s] - q_lens[s] + last_tok, s, t))
     large.sort(key=lambda x: -x[0])                       # longest first
     if even is not None:
-        length = {s: n // int(m) for s, n, m in zip(small_ids, n_keys, even)}
-        small.sort(key=lambda x: -length[x[0]])           # (stable: the ranges of a request stay side by side)
+        place = {small_ids[i]: at for at, i in enumerate(longest_first(np.asarray(n_keys, np.int64), even))}
+        small.sort(key=lambda x: place[x[0]])             # (stable: the ranges of a request stay side by side)
     small_arr = np.array(small, np.int32).reshape(-1, 4)
     if fixed_capacity:
         if len(small_arr) > cap:

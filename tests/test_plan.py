@@ -108,3 +108,16 @@ def test_even_ranges_beside_prompt_portions():
     assert busy["max_splits"] == alone["max_splits"] and busy["num_small_tokens"] == alone["num_small_tokens"]
     small = busy["small"].reshape(-1, 4)
     assert set(small[small[:, 0] >= 0][:, 0].tolist()) == set(range(33)) and (alone["small"] == -1).all()
+
+
+@pytest.mark.parametrize("k_lens,nkv,pad", [(list(range(131, 3501, 130)), 8, 32), (list(range(70, 778, 5)), 4, 192), ([3000] * 16, 8, 16)])
+def test_even_ranges_do_not_depend_on_the_step_they_were_planned_for(k_lens, nkv, pad):
+    """A replayed decode step keeps its plan until a context grows past another multiple of 128 keys.  So that it gives what
+    the same step gives with a plan of its own, bit for bit, all lengths between two multiples have one plan."""
+    kw = dict(cluster_max=8, long_keys=600, slots=296, pad_requests=pad, fixed_capacity=True)
+    S = len(k_lens)
+    first, last = [-(-k // 128) * 128 - 127 for k in k_lens], [-(-k // 128) * 128 for k in k_lens]
+    plans = [general([1] * S, lens, 8, nkv, None, **kw) for lens in (k_lens, first, last)]
+    assert plans[0]["even"]
+    for key in ("small", "splits"):
+        assert np.array_equal(plans[0][key], plans[1][key]) and np.array_equal(plans[0][key], plans[2][key]), key
