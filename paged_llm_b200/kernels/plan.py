@@ -70,6 +70,8 @@ def even_max_splits(scratch_rows: int, max_splits: int) -> int:
 # Contexts are rounded up to multiples of this many keys before they are cut: a plan then changes only when a context grows
 # past another multiple, which is when a replayed step makes its plan anew, and never depends on the step it was made for.
 GRAIN = 128
+# Lengths of a range that `split_evenly` weighs, in even shares; the first stands for the longest context.
+RANGE_LENGTHS = np.array([[1.0], [1.0], [1.15], [1.35], [1.6], [2.0], [2.7], [4.0]])
 
 
 def split_evenly(keys: np.ndarray, extra: int, max_splits: int) -> np.ndarray:
@@ -77,25 +79,41 @@ def split_evenly(keys: np.ndarray, extra: int, max_splits: int) -> np.ndarray:
     (131 to 3,500 keys in one batch: a block per request and kv head walks 3,500 keys alone while most others have long
     ended).  `extra` ranges per kv head are resident at a time, and fit the lists beside one per request; of a few lengths
     of a range, none below an even share, the one after which the last block should end first."""
-    keys = -(-keys // GRAIN) * GRAIN
-    total, longest = int(keys.sum()), int(keys.max())
-    share = max(GRAIN, -(-total // extra))
-    best = None
-    for length in [longest] + [int(share * f) for f in (1.0, 1.15, 1.35, 1.6, 2.0, 2.7, 4.0)]:
-        ns = np.clip(-(-keys // length), 1, max_splits)
-        cost = -(-keys // ns) + BLOCK_KEYS + MERGE_KEYS * (ns > 1)
-        # the last block ends no earlier than an even share, nor than k + 1 blocks of which a place must take that many
-        blocks = np.sort(np.repeat(cost, ns))[::-1]
-        at = blocks[::extra]
-        end = max(int(blocks.sum()) / extra, int((at * np.arange(1, len(at) + 1)).max()))
-        if best is None or end < best[0]:
-            best = (end, ns)
-    return best[1].astype(np.int32)
+    keys = (keys + (GRAIN - 1)) // GRAIN * GRAIN
+    longest = int(keys.max())
+    if longest <= GRAIN:
+        return np.ones(len(keys), np.int32)
+    share = max(GRAIN, -(-int(keys.sum()) // extra))
+    # all lengths at once, a row each
+    length = (share * RANGE_LENGTHS).astype(np.int64)
+    length[0, 0] = longest
+    ns = np.minimum((keys + (length - 1)) // length, max_splits)
+    cost = (keys + (ns - 1)) // ns + BLOCK_KEYS + MERGE_KEYS * (ns > 1)
+    # the blocks by falling cost (cost and number of a request's ranges in one word, so that one sort does), and how many
+    # come up to each: the last block ends no earlier than an even share, nor than k blocks of which a place must take that many
+    order = np.sort((-cost << 16) + ns, axis=1)
+    cost, many = -(order >> 16), order & 0xFFFF
+    upto = np.cumsum(many, axis=1)
+    end = np.maximum((cost * many).sum(1) / extra, ((upto + (extra - 1)) // extra * cost).max(1))
+    return ns[int(end.argmin())].astype(np.int32)
 
 
-def longest_first(keys: np.ndarray, ns: np.ndarray) -> np.ndarray:
-    """Order of the requests of such a step in its list: by the length of their ranges."""
-    return np.argsort(-(-(-keys // GRAIN) * GRAIN // ns), kind="stable")
+def even_items(ids: np.ndarray, base: np.ndarray, keys: np.ndarray, ns: np.ndarray, capacity: int | None) -> np.ndarray:
+    """The list of such a step: the ranges of a request side by side, requests with long ranges first, filled up with
+    items of no request to `capacity`."""
+    order = np.argsort(-((keys + (GRAIN - 1)) // GRAIN * GRAIN // ns), kind="stable")
+    total = int(ns.sum())
+    if capacity is not None and total > capacity:
+        raise PlanCapacityError(f"{total} small items for a capacity of {capacity}")
+    heads = np.empty((len(ns), 4), np.int32)
+    many = ns[order]
+    heads[:, 0], heads[:, 1], heads[:, 3] = ids[order], base[order], many
+    heads[:, 2] = many - np.cumsum(many)                  # minus the place of the request's first range
+    small = np.empty((capacity if capacity is not None else total, 4), np.int32)
+    small[:total] = np.repeat(heads, many, axis=0)
+    small[:total, 2] += np.arange(total, dtype=np.int32)
+    small[total:] = -1
+    return small
 
 
 def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_splits, fixed_capacity,
@@ -110,20 +128,12 @@ def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_sp
         lk = np.asarray(k_lens, np.int64)
         most = even_max_splits(n_req, max_splits)
         ns = split_evenly(lk, extra, most)
-        order = longest_first(lk, ns).astype(np.int32)
-        many = ns[order]
-        first = np.cumsum(many) - many
-        total = int(ns.sum())
-        small = np.empty((total, 4), np.int32)
-        small[:, 0] = small[:, 1] = np.repeat(order, many)
-        small[:, 2] = np.arange(total, dtype=np.int32) - np.repeat(first, many).astype(np.int32)
-        small[:, 3] = np.repeat(many, many)
+        ids = np.arange(S, dtype=np.int32)                                       # (the scratch base too: one token each)
+        small = even_items(ids, ids, lk, ns, S_pad + extra if fixed_capacity else None)
         splits = np.ones((S_pad, 2), np.int32)
         splits[:, 1] = 0
         splits[:S, 0] = ns
-        splits[:S, 1] = np.arange(S, dtype=np.int32)
-        if fixed_capacity:
-            small = np.concatenate([small, np.full((S_pad + extra - total, 4), -1, np.int32)])
+        splits[:S, 1] = ids
         return {"small": small.reshape(-1), "large": np.zeros(0, np.int32), "splits": splits.reshape(-1),
                 "max_splits": int(most if fixed_capacity else ns.max()),
                 "num_small_tokens": int(S_pad if fixed_capacity else S), "long_context": long_context, "even": True}
@@ -204,18 +214,24 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
         want = even_max_splits(S_pad * max(1, small_rows // group_size) if fixed_capacity else len(small_ids), max_splits)
         cap = S_pad + extra
     n_keys = [visible_keys(k_lens[s] - q_lens[s], k_lens[s], window, chunk, keep_first) for s in small_ids]
-    even = split_evenly(np.asarray(n_keys, np.int64), extra, want) if extra and small_ids else None
     splits = np.ones((S_pad, 2), np.int32)
     splits[:, 1] = 0
     small = []
+    small_arr = None
     scratch_base = 0
-    for i, s in enumerate(small_ids):
-        nq = q_lens[s]
-        ns = int(even[i]) if extra else max(1, min(want, -(-n_keys[i] // min_split_keys)))
-        splits[s] = (ns, scratch_base)
-        for j in range(ns):
-            small.append((s, scratch_base, j, ns))
-        scratch_base += nq
+    if extra and small_ids:
+        ids, keys, new = np.array(small_ids), np.array(n_keys, np.int64), np.array([q_lens[s] for s in small_ids])
+        ns, upto = split_evenly(keys, extra, want), np.cumsum(new)
+        splits[ids, 0], splits[ids, 1] = ns, upto - new
+        scratch_base = int(upto[-1])
+        small_arr = even_items(ids, upto - new, keys, ns, cap if fixed_capacity else None)
+    else:
+        for s, n in zip(small_ids, n_keys):
+            ns = max(1, min(want, -(-n // min_split_keys)))
+            splits[s] = (ns, scratch_base)
+            for j in range(ns):
+                small.append((s, scratch_base, j, ns))
+            scratch_base += q_lens[s]
     large = []
     for s in range(S):
         rows = q_lens[s] * group_size
@@ -226,10 +242,8 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
             last_tok = min(rows - 1, (t + 1) * large_rows - 1) // group_size
             large.append((k_lens[s] - q_lens[s] + last_tok, s, t))
     large.sort(key=lambda x: -x[0])                       # longest first
-    if even is not None:
-        place = {small_ids[i]: at for at, i in enumerate(longest_first(np.asarray(n_keys, np.int64), even))}
-        small.sort(key=lambda x: place[x[0]])             # (stable: the ranges of a request stay side by side)
-    small_arr = np.array(small, np.int32).reshape(-1, 4)
+    if small_arr is None:
+        small_arr = np.array(small, np.int32).reshape(-1, 4)
     if fixed_capacity:
         if len(small_arr) > cap:
             raise PlanCapacityError(f"{len(small_arr)} small items for a capacity of {cap}")
