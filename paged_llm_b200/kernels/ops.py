@@ -1324,7 +1324,7 @@ class CudaOps:
             large_rows=self._large_rows(head_dim), min_split_keys=self.MIN_SPLIT_KEYS, num_sms=self.num_sms,
             max_splits=self.MAX_SPLITS, pad_requests=pad_requests, fixed_capacity=fixed_capacity,
             cluster_max=self.MAX_CLUSTER if self.cluster_attention else 0, long_keys=self.CLUSTER_KEYS,
-            pad_tokens=pad_tokens, slots=self._attention_slots(head_dim))
+            pad_tokens=pad_tokens, slots=self._attention_slots(head_dim), head_dim=head_dim)
 
     def _attention_slots(self, head_dim: int) -> int:
         """Blocks of the decode kernel that are resident at a time, two per SM (0: its ranges are not cut evenly)."""

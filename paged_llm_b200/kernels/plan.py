@@ -61,10 +61,15 @@ def even_ranges(num_requests: int, num_kv_heads: int, num_sms: int, slots: int, 
     return max(1, slots // max(num_kv_heads, 1))
 
 
-def even_max_splits(scratch_rows: int, max_splits: int) -> int:
-    """Ranges a request may have in such a step: bounded so that the scratch for the partial results stays small (at 32
-    heads of 64 some 17 MB)."""
-    return int(max(4, min(max_splits, 2048 // max(scratch_rows, 1))))
+# Scratch for the partial results of such a step: bytes, and (row, range) pairs.
+EVEN_SCRATCH_BYTES, EVEN_SCRATCH_ROWS = 36 << 20, 2048
+
+
+def even_max_splits(scratch_rows: int, num_heads: int, head_dim: int, max_splits: int) -> int:
+    """Ranges a request may have in such a step: as many as EVEN_SCRATCH_ROWS and EVEN_SCRATCH_BYTES have room for (a row and
+    range takes a maximum, a sum and `head_dim` values of 4 bytes per query head), one if they have room for less."""
+    rows = max(scratch_rows, 1)
+    return int(max(1, min(max_splits, EVEN_SCRATCH_ROWS // rows, EVEN_SCRATCH_BYTES // (rows * num_heads * (head_dim + 2) * 4))))
 
 
 # Contexts are rounded up to multiples of this many keys before they are cut: a plan then changes only when a context grows
@@ -117,7 +122,7 @@ def even_items(ids: np.ndarray, base: np.ndarray, keys: np.ndarray, ns: np.ndarr
 
 
 def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_splits, fixed_capacity,
-                 cluster_max=0, long_keys=0, slots=0) -> dict:
+                 cluster_max=0, long_keys=0, slots=0, num_heads=32, head_dim=64) -> dict:
     """The same plan for the common step in which every request brings one token, in array form."""
     n_req = S_pad if fixed_capacity else S
     long_context = is_long_context(n_req, num_kv_heads, num_sms, max_splits, cluster_max, long_keys,
@@ -126,7 +131,7 @@ def _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_sp
         else even_ranges(n_req, num_kv_heads, num_sms, slots, max_splits)
     if extra:
         lk = np.asarray(k_lens, np.int64)
-        most = even_max_splits(n_req, max_splits)
+        most = even_max_splits(n_req, num_heads, head_dim, max_splits)
         ns = split_evenly(lk, extra, most)
         ids = np.arange(S, dtype=np.int32)                                       # (the scratch base too: one token each)
         small = even_items(ids, ids, lk, ns, S_pad + extra if fixed_capacity else None)
@@ -192,9 +197,10 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
                    large_rows: int, min_split_keys: int, num_sms: int, max_splits: int = 32,
                    pad_requests: int | None = None, fixed_capacity: bool = False, cluster_max: int = 0,
                    long_keys: int = 0, pad_tokens: int | None = None, chunk: int | None = None,
-                   keep_first: int | None = None, slots: int = 0) -> dict:
+                   keep_first: int | None = None, slots: int = 0, head_dim: int = 64) -> dict:
     """`slots` > 0 (blocks that are resident at a time): steps of so many requests that none would be split, and
-    long-context steps, are cut into ranges of about equal length instead (see `split_evenly`).
+    long-context steps, are cut into ranges of about equal length instead (see `split_evenly`; `head_dim` says what the
+    scratch for their partial results takes).
 
     `pad_tokens` (with `fixed_capacity`, for a step of mixed items that replays a captured graph): both lists
     get the capacity of any step of that many tokens and `pad_requests` requests, filled up with items of
@@ -203,7 +209,7 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
     S_pad = pad_requests or S
     if pad_tokens is None and S and max(q_lens) == 1 and group_size <= small_rows and not window and not chunk:
         return _plan_decode(S, S_pad, k_lens, num_kv_heads, min_split_keys, num_sms, max_splits, fixed_capacity,
-                            cluster_max, long_keys, slots)
+                            cluster_max, long_keys, slots, group_size * num_kv_heads, head_dim)
     small_ids = [s for s in range(S) if q_lens[s] * group_size <= small_rows]
     n_small = S_pad if fixed_capacity else len(small_ids)
     want = wanted_splits(n_small, num_kv_heads, num_sms, max_splits)
@@ -211,7 +217,8 @@ def plan_attention(q_lens, k_lens, group_size: int, num_kv_heads: int, window: i
     # (what a captured graph has baked in depends on its capacity alone, also where no request is small this time)
     extra = even_ranges(n_small, num_kv_heads, num_sms, slots, max_splits) if n_small else 0
     if extra:
-        want = even_max_splits(S_pad * max(1, small_rows // group_size) if fixed_capacity else len(small_ids), max_splits)
+        want = even_max_splits(S_pad * max(1, small_rows // group_size) if fixed_capacity else sum(q_lens[s] for s in small_ids),
+                               group_size * num_kv_heads, head_dim, max_splits)
         cap = S_pad + extra
     n_keys = [visible_keys(k_lens[s] - q_lens[s], k_lens[s], window, chunk, keep_first) for s in small_ids]
     splits = np.ones((S_pad, 2), np.int32)

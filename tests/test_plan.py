@@ -165,3 +165,21 @@ def test_even_ranges_cost_the_host_little_more_than_equal_ones(S, pad):
         return least
 
     assert best(296) < 5 * best(0)
+
+
+@pytest.mark.parametrize("nh,nkv,d", [(32, 4, 64), (32, 8, 128), (32, 32, 128), (64, 64, 256), (128, 8, 128), (16, 16, 16)])
+def test_even_ranges_keep_the_scratch_within_its_bound(nh, nkv, d):
+    """What the partial results of any even step take, replayed or not, decoding alone or mixed: the declared bound, or what
+    one range per request takes where that is more."""
+    G, kw = nh // nkv, dict(cluster_max=8, long_keys=600, slots=296)
+    for pad in (8, 64, 160, 256):
+        steps = [([1] * pad, dict(pad_requests=pad, fixed_capacity=True)), ([1] * pad, {}),
+                 ([1] * (pad - 1) + [256], dict(pad_requests=pad, fixed_capacity=True, pad_tokens=512)),
+                 ([1] * (pad - 1) + [max(1, 16 // G)], {})]
+        for q_lens, more in steps:
+            plan = general(q_lens, [4000] * pad, G, nkv, None, head_dim=d, **kw, **more)
+            rows = max(plan["num_small_tokens"], 1)
+            splits = plan["splits"].reshape(-1, 2)
+            assert plan["max_splits"] >= splits[:, 0].max()
+            if plan["even"] and plan["max_splits"] > 1:
+                assert rows * nh * plan["max_splits"] * (d + 2) * 4 <= planning.EVEN_SCRATCH_BYTES
