@@ -1351,10 +1351,10 @@ class CudaOps:
                     and max(ctx.host.q_lens) * (nh // nkv) <= self.SMALL_ROWS and not plan.long_context
                     and not plan.even)
 
-    @staticmethod
-    def _rotates_inside(plan, ctx) -> bool:
+    def _rotates_inside(self, plan, ctx, nh: int, nkv: int) -> bool:
         """A decode step whose ranges were cut evenly: the list form rotates and writes the cache as the clusters do."""
-        return bool(plan.even and plan.n_small and not plan.n_large and max(ctx.host.q_lens) == 1)
+        return bool(plan.even and plan.n_small and not plan.n_large
+                    and max(ctx.host.q_lens) * (nh // nkv) <= self.SMALL_ROWS)
 
     def qkv_attention(self, h, w_qkv, nh, nkv, d, position, ctx, kv, block_table, scale, window, write=True,
                       softcap=None, slopes=None, chunk=None, value_from_key=False) -> torch.Tensor:
@@ -1370,7 +1370,7 @@ class CudaOps:
                   and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens
                   and not self._skinny_ok(h, (nh + 2 * nkv) * d) and self.compute_dtype == torch.bfloat16
                   and kv.dtype == torch.bfloat16
-                  and (self._runs_as_clusters(plan, ctx, nh, nkv, True) or self._rotates_inside(plan, ctx))
+                  and (self._runs_as_clusters(plan, ctx, nh, nkv, True) or self._rotates_inside(plan, ctx, nh, nkv))
                   and self.rope_in_attention)
         if inside:
             qkv = self.linear(h, w_qkv)
@@ -1434,7 +1434,7 @@ class CudaOps:
             lib, fn = self.core, self.core.pl_attention_f32
         p.cluster = 0
         if rope is not None:
-            if not (bf16 and (self._runs_as_clusters(plan, ctx, nh, nkv, bf16) or self._rotates_inside(plan, ctx))) or softcap or slopes is not None or dist_bias is not None or keep_first:
+            if not (bf16 and (self._runs_as_clusters(plan, ctx, nh, nkv, bf16) or self._rotates_inside(plan, ctx, nh, nkv))) or softcap or slopes is not None or dist_bias is not None or keep_first:
                 raise KernelError("rotary positions inside the attention kernel: only for decode steps that run as "
                                   "clusters or in even ranges, without score modifiers")
             assert qkv.shape[1] == (nh + 2 * nkv) * d and rope.table.is_contiguous() and rope.rotary_dim == d

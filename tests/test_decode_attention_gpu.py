@@ -79,3 +79,67 @@ def test_even_ranges_against_plain_attention(ops, nh, nkv, d, ps, S, pad):
         # probabilities and the result are rounded to bfloat16 (2^-9 each), relative to values of up to 4.5
         torch.testing.assert_close(out[s], want, atol=2 * 4.5 * 2 ** -9, rtol=2 ** -8, msg=f"request {s} of {n} keys")
     assert ops.kernel_timeouts() == 0
+
+
+@pytest.mark.parametrize("nq", [1, 2])
+@pytest.mark.parametrize("nh,nkv,d,ps,window", [(32, 8, 64, 16, None), (32, 8, 128, 16, None),             # attention_decode.cuh
+                                                (4, 4, 16, 16, None), (8, 4, 32, 16, None), (6, 2, 48, 16, None), (8, 2, 80, 16, None),
+                                                (4, 2, 256, 16, None), (16, 2, 64, 8, None), (8, 2, 128, 20, None),
+                                                (16, 2, 64, 16, 50), (4, 4, 16, 8, 300), (4, 2, 256, 16, 200)])
+def test_rotation_inside_the_list_form(ops, nh, nkv, d, ps, window, nq):
+    """The list form that rotates and writes the cache itself, for every kernel behind it (head sizes, page sizes, windows),
+    one and two new tokens per request.  At 385 and 897 keys the last range begins with the second of the two."""
+    from paged_llm_b200.engine.context import AttentionPlan, HostBatch
+    G, W = nh // nkv, (nh + 2 * nkv) * d
+    k_lens = [n for n in [2, 3, 16, 17, 31, 32, 33, 34, 127, 128, 129, 144, 385, 513, 897, 1000, 2049] if n >= nq] * 2
+    S, T = len(k_lens), len(k_lens) * nq
+    g = torch.Generator(device="cuda").manual_seed(d + nq)
+    pages = [-(-n // ps) for n in k_lens]
+    order = torch.randperm(sum(pages) + 3, generator=torch.Generator().manual_seed(1)).int()
+    bt = torch.full((S, max(pages) + 1), 10 ** 6, dtype=torch.int32)
+    kv = torch.full((sum(pages) + 3, 2, nkv, ps, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    qkv = torch.randn(T, W, device="cuda", generator=g).to(torch.bfloat16)
+    table = torch.randn(4096, d // 2, 2, device="cuda", generator=g)
+    old, o = [], 0
+    for s, n in enumerate(k_lens):                        # all keys but the step's own are in the cache, the rest is NaN
+        mine = order[o:o + pages[s]]
+        bt[s, :pages[s]] = mine
+        o += pages[s]
+        both = torch.randn(2, n - nq, nkv, d, device="cuda", generator=g).to(torch.bfloat16)
+        flat = torch.full((2, pages[s] * ps, nkv, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        flat[:, :n - nq] = both
+        kv[mine.long().cuda()] = flat.view(2, pages[s], ps, nkv, d).permute(1, 0, 3, 2, 4)
+        old.append(both)
+    before = kv.clone()
+    splits = [min(8, -(-n // 128)) for n in k_lens]
+    small = np.array([(s, s * nq, j, m) for s, m in enumerate(splits) for j in range(m)], np.int32)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.int32)).cuda()
+    ap = AttentionPlan(dev(small), None, dev([(m, s * nq) for s, m in enumerate(splits)]), len(small), 0, 8, T, False, True)
+    host = HostBatch([nq] * S, [n - nq for n in k_lens], [-1] * S)
+    key = (G, nkv, window, d)
+    ctx = types.SimpleNamespace(num_tokens=T, num_seqs=S, host=host, cu_seqlens_q=dev(host.cu), seq_lens_k=dev(k_lens),
+                                attention_plans={key: ap}, padded=False)
+    rope = types.SimpleNamespace(table=table, rotary_dim=d)
+    for _ in range(2):                                    # the second time finds the counters as the first left them
+        launches = ops.launches
+        out = ops.paged_attention(qkv, nh, nkv, d, kv, bt.cuda(), ctx, d ** -0.5, window, rope=rope).float()
+        assert ops.launches == launches + 1
+    for s, n in enumerate(k_lens):
+        keys, vals = old[s][0], old[s][1]
+        for i in range(nq):
+            q, k, v = (t.view(-1, d) for t in qkv[s * nq + i].split([nh * d, nkv * d, nkv * d]))
+            pos = n - nq + i
+            q, k = rotated(q, table[pos]), rotated(k, table[pos])
+            slot = kv[bt[s, pos // ps], :, :, pos % ps]
+            before[bt[s, pos // ps], :, :, pos % ps] = slot
+            # (the kernel may round one product of a rotated pair less than torch does: a neighbouring bfloat16)
+            torch.testing.assert_close(slot[0].float(), k.float(), atol=2 ** -20, rtol=2 ** -7, msg=f"request {s}: the cached key")
+            assert torch.equal(slot[1], v), f"request {s}: the cached value"
+            keys, vals = torch.cat([keys, slot[0][None]]), torch.cat([vals, v[None]])
+            lo = max(0, pos - window + 1) if window else 0
+            score = torch.einsum("jgd,njd->jgn", q.float().view(nkv, G, d), keys[lo:].float()) * d ** -0.5
+            want = torch.einsum("jgn,njd->jgd", score.softmax(-1), vals[lo:].float()).reshape(-1)
+            # probabilities and the result are rounded to bfloat16 (2^-9 each), relative to values of up to 4.5
+            torch.testing.assert_close(out[s * nq + i], want, atol=2 * 4.5 * 2 ** -9, rtol=2 ** -8, msg=f"request {s} of {n} keys")
+    assert ((kv == before) | (torch.isnan(kv) & torch.isnan(before))).all(), "only the slots of the step's own tokens may change"
+    assert ops.kernel_timeouts() == 0
