@@ -143,3 +143,54 @@ def test_rotation_inside_the_list_form(ops, nh, nkv, d, ps, window, nq):
             torch.testing.assert_close(out[s * nq + i], want, atol=2 * 4.5 * 2 ** -9, rtol=2 ** -8, msg=f"request {s} of {n} keys")
     assert ((kv == before) | (torch.isnan(kv) & torch.isnan(before))).all(), "only the slots of the step's own tokens may change"
     assert ops.kernel_timeouts() == 0
+
+
+@pytest.mark.parametrize("nh,nkv,d,H", [(32, 8, 64, 1280), (32, 8, 128, 96), (8, 8, 16, 96), (8, 8, 48, 1280), (8, 4, 256, 64), (32, 4, 64, 2048)])
+@pytest.mark.parametrize("q_lens", [[1] * 40, [1] * 64, [2, 1, 2] * 14])
+def test_front_of_a_decode_step_as_it_is_planned(ops, nh, nkv, d, H, q_lens):
+    """`qkv_attention` of a step whose ranges the plan cuts evenly, as the engine runs it: the product (this package's or the
+    library's, by width), then one kernel that rotates, writes the cache and attends.  Held to the same pieces in float32."""
+    from paged_llm_b200.parts.rope import RotaryEncoding
+    from tests import plain_llama
+    from tests.test_kernels_gpu import make_ctx, paged_case, tol
+    dtype, ps, G = torch.bfloat16, 16, nh // nkv
+    S, T = len(q_lens), sum(q_lens)
+    k_lens = [EDGES[(i * 5) % len(EDGES)] + 2 for i in range(S)]
+    rope = RotaryEncoding({}, head_dim=d, theta=10000.0)
+    rope.prepare(4096, "cuda", ops)
+    _, kv, bt, keys, vals = paged_case(q_lens, k_lens, nh, nkv, d, ps, dtype, seed=3)
+    g = torch.Generator().manual_seed(d)
+    h = torch.randn(T, H, generator=g).to(dtype)
+    w = (torch.randn((nh + 2 * nkv) * d, H, generator=g) * H ** -0.5).to(dtype)
+    y = (h.float() @ w.float().T).to(dtype).float()                       # the projection rounds to bfloat16
+    pos = torch.cat([torch.arange(k - q, k) for q, k in zip(q_lens, k_lens)])
+    cos, sin = plain_llama.rotary_cos_sin(pos, plain_llama.inv_frequencies(d, 10000.0, None))
+    q_rot = plain_llama.apply_rotary(y[:, :nh * d].view(T, nh, d), cos, sin).to(dtype).float()
+    k_rot = plain_llama.apply_rotary(y[:, nh * d:(nh + nkv) * d].view(T, nkv, d), cos, sin).to(dtype).float()
+    v_new = y[:, (nh + nkv) * d:].view(T, nkv, d)
+    ctx = make_ctx(ops, q_lens, k_lens, nh, nkv, None, d, planned=True)
+    plan = ctx.attention_plans[(G, nkv, None, d)]
+    inside = max(q_lens) * G <= 16
+    if nkv * S >= 148:
+        assert plan.even and not ops._runs_as_clusters(plan, ctx, nh, nkv, True) and ops._rotates_inside(plan, ctx, nh, nkv) == inside
+    kv_dev = kv.cuda()
+    at = ctx.host.cu
+    for s in range(S):
+        for n in range(k_lens[s] - q_lens[s], k_lens[s]):                 # poison until the step writes them
+            kv_dev[bt[s, n // ps], :, :, n % ps] = float("nan")
+            t = at[s] + n - (k_lens[s] - q_lens[s])
+            keys[s][n], vals[s][n] = k_rot[t], v_new[t]
+    before = ops.launches
+    out = ops.qkv_attention(h.cuda(), w.cuda(), nh, nkv, d, rope, ctx, kv_dev, bt.cuda(), d ** -0.5, None).float().cpu()
+    if inside:
+        assert ops.launches - before == 1 + (H >= 1280 and T <= 64)
+    for s, (nq, n) in enumerate(zip(q_lens, k_lens)):
+        for j in range(n - nq, n):
+            t = at[s] + j - (n - nq)
+            score = torch.einsum("jgd,njd->jgn", q_rot[t].view(nkv, G, d), keys[s][:j + 1]) * d ** -0.5
+            want = torch.einsum("jgn,njd->jgd", score.softmax(-1), vals[s][:j + 1]).reshape(-1)
+            torch.testing.assert_close(out[t], want, atol=tol(dtype), rtol=tol(dtype), msg=f"request {s} of {n} keys")
+            got = kv_dev[bt[s, j // ps], :, :, j % ps].float().cpu()
+            torch.testing.assert_close(got[0], keys[s][j], atol=tol(dtype), rtol=tol(dtype))
+            torch.testing.assert_close(got[1], vals[s][j], atol=tol(dtype), rtol=tol(dtype))
+    assert ops.kernel_timeouts() == 0

@@ -186,7 +186,8 @@ def paged_case(q_lens, k_lens, nh, nkv, d, ps, dtype, seed=0, spare=3):
     return q, kv.to(dtype), bt, keys, vals
 
 
-def make_ctx(ops, q_lens, k_lens, nh, nkv, window, d=64):
+def make_ctx(ops, q_lens, k_lens, nh, nkv, window, d=64, planned=False):
+    """`planned`: the step takes the form that its plan says, as in the engine (else clusters wherever they can run it)."""
     from paged_llm_b200.engine.context import AttentionPlan, HostBatch
     S = len(q_lens)
     host = HostBatch(list(q_lens), [k - q for q, k in zip(q_lens, k_lens)], [-1] * S)
@@ -194,7 +195,8 @@ def make_ctx(ops, q_lens, k_lens, nh, nkv, window, d=64):
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.int32)).cuda()
     small, large = plan["small"].reshape(-1, 4), plan["large"].reshape(-1, 4)
     ap = AttentionPlan(dev(small) if len(small) else None, dev(large) if len(large) else None, dev(plan["splits"]),
-                       len(small), len(large), plan["max_splits"], plan["num_small_tokens"])
+                       len(small), len(large), plan["max_splits"], plan["num_small_tokens"],
+                       planned and plan["long_context"], planned and plan["even"])
     T = sum(q_lens)
     pos = np.concatenate([np.arange(k - q, k) for q, k in zip(q_lens, k_lens)])
     tseq = np.concatenate([np.full(q, s) for s, q in enumerate(q_lens)])
