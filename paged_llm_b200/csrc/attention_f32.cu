@@ -249,11 +249,12 @@ int pl_attn_check(const AttnParams& p, const char* who) {
 template <int NC> static int launch_attn_f32(const AttnParams& p, cudaStream_t stream) {
     const size_t smem = ((size_t)F32_ROWS * p.d + 4 * F32_KEYS * 4 + F32_STAGES * F32_KEYS * (2 * p.d + 4)) * sizeof(float);
     constexpr size_t most = ((size_t)F32_ROWS * 64 * NC + 4 * F32_KEYS * 4 + F32_STAGES * F32_KEYS * (2 * 64 * NC + 4)) * sizeof(float);
-    static bool attr_set = false;
-    if (!attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(attn_f32_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-        attr_set = true;
-    }
+    static PerDevice<char> ready;
+    if (!ready.get("attention_f32", [&](char&) {
+            PL_CUDA(cudaFuncSetAttribute(attn_f32_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+            return 0;
+        }))
+        return 1;
     PL_CUDA(launch_pdl(attn_f32_kernel<NC>, dim3(p.n_work * p.nkv), dim3(128), smem, stream, p));
     return 0;
 }

@@ -9,6 +9,9 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+#include <mutex>
+
 #define PL_EXPORT extern "C" __attribute__((visibility("default")))
 
 enum PlDtype { PL_F32 = 0, PL_BF16 = 1 };
@@ -31,6 +34,35 @@ int pl_fail(const char* fmt, ...);
         cudaError_t e__ = (expr);                                                \
         if (e__ != cudaSuccess) return pl_fail("%s: %s", #expr, cudaGetErrorString(e__)); \
     } while (0)
+
+// What a launcher sets or finds out once per device of the process (function attributes belong to a device), whichever
+// thread comes first.
+template <typename T> class PerDevice {
+    static constexpr int MAX_DEVICES = 64;
+    std::mutex mu;
+    std::atomic<bool> known[MAX_DEVICES] = {};
+    T value[MAX_DEVICES] = {};
+
+  public:
+    // The current device's value; `make(T&)` fills it in the first time and returns 0, or the code of an error that it
+    // recorded.  Null with the error recorded.
+    template <typename F> const T* get(const char* who, F make) {
+        int dev = 0;
+        const cudaError_t rc = cudaGetDevice(&dev);
+        if (rc != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
+            pl_fail("%s: device index %d: %s", who, dev, rc != cudaSuccess ? cudaGetErrorString(rc) : "out of range");
+            return nullptr;
+        }
+        if (!known[dev].load(std::memory_order_acquire)) {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!known[dev].load(std::memory_order_relaxed)) {
+                if (make(value[dev]) != 0) return nullptr;
+                known[dev].store(true, std::memory_order_release);
+            }
+        }
+        return &value[dev];
+    }
+};
 
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }

@@ -198,11 +198,12 @@ template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool VEC>
 int launch_sgemm(const SgemmParams& p, int serial_from, cudaStream_t stream) {
     constexpr int stages = STAGES * (BM + BN) * (BK + 4) * 4, tile = BM * BN * 4;
     static_assert(stages >= tile, "a part's sums fit where the stages were");
-    static bool attr_set = false;
-    if (!attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(sgemm_nt_kernel<BM, BN, TM, TN, BK, STAGES, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, stages + tile));
-        attr_set = true;
-    }
+    static PerDevice<char> ready;
+    if (!ready.get("gemm_f32", [&](char&) {
+            PL_CUDA(cudaFuncSetAttribute(sgemm_nt_kernel<BM, BN, TM, TN, BK, STAGES, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, stages + tile));
+            return 0;
+        }))
+        return 1;
     const int parts = (p.K + p.part_len - 1) / p.part_len;
     const long long tiles = (long long)((p.N + BN - 1) / BN) * ((p.M + BM - 1) / BM);
     cudaLaunchConfig_t cfg = {};

@@ -4,7 +4,8 @@
 // What bounds it is the read of W, so the machine is filled with readers of W: a block takes 128 rows of W (the 128 lanes
 // of the accumulator; the tokens are its columns, so a tile is never wider than the step) and one part of k; the blocks of
 // a cluster share the rows and add their parts up through distributed shared memory, each for its own tokens, in a fixed
-// order.  The number of parts depends on N and K alone: a token's result does not depend on the batch.  Two blocks fit an
+// order.  The number of parts depends on the product (N, K, what follows it) and the GPU alone: a token's result does not
+// depend on the batch.  Two blocks fit an
 // SM, so the copies of one run on while the other drains, and since W does not depend on the kernel in front, a block
 // fills its ring with W before it waits for that kernel and adds the X boxes afterwards.
 //
@@ -282,7 +283,10 @@ template <int EPI> int launch_mid(MidParams p, const void* X, int ldx, const voi
     PL_REQUIRE(p.M >= 1 && p.M <= MID_MAX_COLS && p.N >= 1 && p.K >= MID_BK && p.K % MID_BK == 0 && ldx % 8 == 0,
                "gemm_mid: M=%d (1..%d) N=%d K=%d (a multiple of 64) ldx=%d", p.M, MID_MAX_COLS, p.N, p.K, ldx);
     PL_REQUIRE(p.part_in == nullptr || p.K % 128 == 0, "gemm_mid: a normed input of K=%d", p.K);
-    static int at_once[MID_MAX_PARTS + 1] = {};
+    struct AtOnce {
+        int clusters[MID_MAX_PARTS + 1];
+    };
+    static PerDevice<AtOnce> found;
     constexpr size_t smem = MID_RING + 1024;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(MID_THREADS);
@@ -294,7 +298,7 @@ template <int EPI> int launch_mid(MidParams p, const void* X, int ldx, const voi
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    if (at_once[MID_MAX_PARTS] == 0) {
+    const AtOnce* at_once = found.get("gemm_mid", [&](AtOnce& a) {
         PL_CUDA(cudaFuncSetAttribute(gemm_mid_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         cfg.numAttrs = 1;
         for (int parts = 1; parts <= MID_MAX_PARTS; ++parts) {
@@ -302,9 +306,11 @@ template <int EPI> int launch_mid(MidParams p, const void* X, int ldx, const voi
             cfg.gridDim = dim3(parts);
             int n = 0;
             PL_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_mid_kernel<EPI>, &cfg));
-            at_once[parts] = 2 * n;      // (it counts one block per SM for any kernel with tensor memory; two fit, and two run)
+            a.clusters[parts] = 2 * n;   // (it counts one block per SM for any kernel with tensor memory; two fit, and two run)
         }
-    }
+        return 0;
+    });
+    if (!at_once) return 1;
     p.cols = (p.M + 31) / 32 * 32;
     const int stages = MID_RING / (MID_W_BYTES + p.cols * 128);
     p.stages = stages < MID_MAX_STAGES ? stages : MID_MAX_STAGES;
@@ -314,7 +320,7 @@ template <int EPI> int launch_mid(MidParams p, const void* X, int ldx, const voi
         !tensor_map_bf16(&w_map, W, (unsigned long long)w_rows, (unsigned long long)p.K, (unsigned long long)p.K, 64))
         return 1;
     const int tiles = EPI == MID_SILU ? (p.I + 63) / 64 : (p.N + MID_ROWS - 1) / MID_ROWS;
-    const int parts = mid_parts(tiles, p.K, at_once);
+    const int parts = mid_parts(tiles, p.K, at_once->clusters);
     cfg.gridDim = dim3(tiles * parts);
     attr[0].val.clusterDim.x = parts;
     static const bool no_pdl = getenv("PAGED_LLM_B200_NO_PDL") != nullptr;
