@@ -7,8 +7,13 @@ constexpr int F32_ROWS = 16;     // query rows per block
 constexpr int F32_KEYS = 32;     // keys per iteration: one per lane
 constexpr int F32_STAGES = 2;
 
-__device__ __forceinline__ void f32_copy(float* dst, const float* src, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
+// W floats from `src`, zeros without one (`any`: an address that may be named all the same).
+template <int W> __device__ __forceinline__ void f32_copy(float* dst, const float* src, const float* any) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = src != nullptr ? 4 * W : 0;
+    const float* from = src != nullptr ? src : any;
+    if (W == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(from), "r"(bytes));
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(from), "r"(bytes));
 }
 
 // grid: (items, kv heads); 128 threads = 4 warps, each owning 4 of the 16 rows.  A tile of 32 keys is brought in by
@@ -16,8 +21,9 @@ __device__ __forceinline__ void f32_copy(float* dst, const float* src, int bytes
 // still.  What bounds it is the issue of shared-memory loads, so four rows share each: a lane reads four elements of
 // its key for four rows' dot products, and the four rows' probabilities of a key as one float4 for its two columns of
 // the weighted sum.  Every sum keeps its order (over the head's elements, over the keys).
-// NC: pairs of columns per lane, ceil(d / 64).
-template <int NC>
+// NC: pairs of columns per lane, ceil(d / 64).  VEC: the cache starts on a 16-byte boundary (and so do all rows); copies
+// of 4 bytes where it does not.
+template <int NC, bool VEC>
 __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
     pdl_launch_dependents();
     const int padding = attn_padding_from(p);
@@ -50,14 +56,15 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnParams p) {
         rows[t % F32_STAGES][tid] = src;
     };
     auto load_tile = [&](int t) {
-        const int st = t % F32_STAGES, chunks = d / 4;
+        constexpr int W = VEC ? 4 : 1;
+        const int st = t % F32_STAGES, chunks = d / W;
         float* kd = Ks + st * F32_KEYS * KP;
         float* vd = Vs + st * F32_KEYS * d;
         for (int e = tid; e < F32_KEYS * chunks; e += 128) {
-            const int j = e / chunks, c = (e - j * chunks) * 4;
+            const int j = e / chunks, c = (e - j * chunks) * W;
             const float* src = rows[st][j];
-            f32_copy(kd + j * KP + c, src != nullptr ? src + c : kv, src != nullptr ? 16 : 0);
-            f32_copy(vd + j * d + c, src != nullptr ? src + v_off + c : kv, src != nullptr ? 16 : 0);
+            f32_copy<W>(kd + j * KP + c, src != nullptr ? src + c : nullptr, kv);
+            f32_copy<W>(vd + j * d + c, src != nullptr ? src + v_off + c : nullptr, kv);
         }
     };
     if (tid < F32_KEYS) {
@@ -246,25 +253,28 @@ int pl_attn_check(const AttnParams& p, const char* who) {
     return 0;
 }
 
-template <int NC> static int launch_attn_f32(const AttnParams& p, cudaStream_t stream) {
+template <int NC, bool VEC> static int launch_attn_f32(const AttnParams& p, cudaStream_t stream) {
     const size_t smem = ((size_t)F32_ROWS * p.d + 4 * F32_KEYS * 4 + F32_STAGES * F32_KEYS * (2 * p.d + 4)) * sizeof(float);
     constexpr size_t most = ((size_t)F32_ROWS * 64 * NC + 4 * F32_KEYS * 4 + F32_STAGES * F32_KEYS * (2 * 64 * NC + 4)) * sizeof(float);
     static PerDevice<char> ready;
     if (!ready.get("attention_f32", [&](char&) {
-            PL_CUDA(cudaFuncSetAttribute(attn_f32_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+            PL_CUDA(cudaFuncSetAttribute(attn_f32_kernel<NC, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
             return 0;
         }))
         return 1;
-    PL_CUDA(launch_pdl(attn_f32_kernel<NC>, dim3(p.n_work * p.nkv), dim3(128), smem, stream, p));
+    PL_CUDA(launch_pdl(attn_f32_kernel<NC, VEC>, dim3(p.n_work * p.nkv), dim3(128), smem, stream, p));
     return 0;
+}
+
+template <bool VEC> static int dispatch_attn_f32(const AttnParams& p, cudaStream_t stream) {
+    return p.d <= 64 ? launch_attn_f32<1, VEC>(p, stream) : p.d <= 128 ? launch_attn_f32<2, VEC>(p, stream) : launch_attn_f32<4, VEC>(p, stream);
 }
 
 PL_EXPORT int pl_attention_f32(const AttnParams* params, cudaStream_t stream) {
     AttnParams p = *params;
     if (p.n_work == 0) return 0;
     if (int rc = pl_attn_check(p, "attention_f32")) return rc;
-    PL_REQUIRE(((uintptr_t)p.kv & 15) == 0, "attention_f32: kv must be 16-byte aligned");
-    return p.d <= 64 ? launch_attn_f32<1>(p, stream) : p.d <= 128 ? launch_attn_f32<2>(p, stream) : launch_attn_f32<4>(p, stream);
+    return ((uintptr_t)p.kv & 15) == 0 ? dispatch_attn_f32<true>(p, stream) : dispatch_attn_f32<false>(p, stream);
 }
 
 PL_EXPORT int pl_attention_combine(const AttnParams* params, int out_dtype, cudaStream_t stream) {

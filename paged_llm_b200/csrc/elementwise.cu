@@ -146,8 +146,8 @@ template <typename TB, typename TW, typename TO>
 static int launch_rmsnorm(float* x, const void* branch, const void* w, void* y, int rows, int H, float eps,
                           cudaStream_t stream) {
     const int threads = H >= 4096 ? 512 : (H >= 1024 ? 256 : 128);
-    const bool aligned = (H & 3) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 7) == 0 &&
-                         ((uintptr_t)w & 7) == 0 && ((uintptr_t)branch & 7) == 0;
+    const bool aligned = (H & 3) == 0 && ((uintptr_t)x & 15) == 0 && (uintptr_t)y % (4 * sizeof(TO)) == 0 &&
+                         (uintptr_t)w % (4 * sizeof(TW)) == 0 && (uintptr_t)branch % (4 * sizeof(TB)) == 0;     // of four elements
     int mode = (size_t)H * 4 <= 40 * 1024 ? 1 : 0;
     if (aligned && H <= threads * 4 * NORM_VEC_ITERS) mode = 2;
     PL_CUDA(launch_pdl(rmsnorm_kernel<TB, TW, TO>, dim3(rows), dim3(threads), mode == 1 ? (size_t)H * 4 : 0, stream, x,

@@ -94,6 +94,11 @@ def _check(lib, rc: int) -> None:
         raise KernelError(lib.pl_last_error().decode())
 
 
+def wide(t: torch.Tensor) -> bool:
+    """Whether the tensor starts where 16-byte accesses may (a view at an odd offset need not)."""
+    return t.data_ptr() % 16 == 0
+
+
 def head_dim_build(d: int) -> int:
     if d % 16 or d <= 0:
         raise KernelError(f"head_dim={d}: the attention kernels take head sizes in steps of 16")
@@ -482,8 +487,8 @@ class CudaOps:
         M, K = h.shape
         return (16 < M <= self.mid_tokens and self.mid_widths[0] <= width < self.mid_widths[1]
                 and M * self.mid_width_per_token <= width and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-                and K % 64 == 0 and w.shape[0] % align == 0 and w.is_contiguous()
-                and ((h.scaled is not None and K % 128 == 0) if isinstance(h, LazyNorm) else h.is_contiguous()))
+                and K % 64 == 0 and w.shape[0] % align == 0 and w.is_contiguous() and wide(w)
+                and ((h.scaled is not None and K % 128 == 0) if isinstance(h, LazyNorm) else h.is_contiguous() and wide(h)))
 
     def _mid_args(self, h):
         """(X, its row stride, partial sums, eps) for a product of `gemm_mid.cu`."""
@@ -558,7 +563,7 @@ class CudaOps:
         M, K = h.shape
         N = w.shape[0]
         few = self._skinny_ok(h, N) and N % 16 == 0 and N % 32 == 0
-        mid = not out_float32 and self._mid_ok(h, w, 128, N) and norm_w.is_contiguous()
+        mid = not out_float32 and self._mid_ok(h, w, 128, N) and norm_w.is_contiguous() and wide(norm_w) and wide(x)
         if not isinstance(h, LazyNorm) and (few or mid):
             assert x.dtype == torch.float32 and x.is_contiguous() and x.shape == (M, N) and h.is_contiguous()
             if self._norm_part is None or self._norm_part.numel() < 2 * N:

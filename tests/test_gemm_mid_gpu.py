@@ -77,3 +77,33 @@ def test_add_and_the_norm_behind_it(ops, M, N, K, wdtype):
     want3 = torch.nn.functional.silu(gate) * up
     assert ((got3 - want3).norm() / want3.norm()).item() < 2 ** -6
     assert ops.kernel_timeouts() == 0
+
+
+def shifted(t, by=1):
+    """The same values at an address that is no multiple of 16 bytes."""
+    buf = torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)
+    out = buf[by:].view(t.shape)
+    out.copy_(t)
+    assert out.data_ptr() % 16 and out.is_contiguous()
+    return out
+
+
+@pytest.mark.parametrize("by", [1, 2])
+@pytest.mark.parametrize("which", ["h", "w", "norm", "norm32", "stream"])
+def test_operands_that_do_not_start_on_16_bytes(ops, which, by):
+    """Views at odd offsets take the library's product, as they did before there was another."""
+    M, N, K = 24, 256, 512
+    h, w, x = randn(M, K, seed=5), randn(N, K, seed=6, std=0.05), randn(M, N, seed=7, dtype=torch.float32)
+    nw = randn(N, seed=8, std=0.1, dtype=torch.float32).add(1)
+    nw = nw if which == "norm32" else nw.to(torch.bfloat16)
+    branch = (h.float() @ w.float().T)
+    want = x + branch
+    h, w, nw, x = (shifted(t, by) if which.startswith(name) else t for name, t in (("h", h), ("w", w), ("norm", nw), ("stream", x)))
+    got = ops.materialize(ops.linear_add_rms_norm(h, w, x, nw, 1e-5)).float()
+    torch.testing.assert_close(x, want, atol=2 ** -8 * float(branch.abs().max()), rtol=1e-6)
+    normed = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-5) * nw.float()
+    torch.testing.assert_close(got, normed, atol=2 ** -6, rtol=2 ** -7)
+    close(ops.linear(h, w), branch, K)
+    gate, up = branch.to(torch.bfloat16).float().chunk(2, 1)
+    act = torch.nn.functional.silu(gate) * up
+    torch.testing.assert_close(ops.gated_act_linear(h, w).float(), act, atol=2 ** -7 * float(act.abs().mean()) + 1e-5, rtol=2 ** -6)

@@ -284,6 +284,22 @@ def test_decode_attention_as_clusters_and_from_the_work_list(ops, cluster, windo
         torch.testing.assert_close(out[cu[s]:cu[s + 1]], want, atol=tol(dtype), rtol=tol(dtype), msg=f"request {s}")
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(8, 2, 64), (4, 2, 128), (4, 1, 256), (6, 2, 48)])
+def test_float32_attention_over_a_cache_that_does_not_start_on_16_bytes(ops, nh, nkv, d):
+    """A cache that is a view at an odd offset gives what an aligned one gives, bit for bit."""
+    q_lens, k_lens, ps = [40, 1, 3], [40, 300, 65], 8
+    ops.set_compute_dtype(torch.float32)
+    q, kv, bt, _, _ = paged_case(q_lens, k_lens, nh, nkv, d, ps, torch.float32, seed=d)
+    ctx = make_ctx(ops, q_lens, k_lens, nh, nkv, None, d)
+    qkv = torch.cat([q.reshape(-1, nh * d), torch.zeros(q.shape[0], 2 * nkv * d)], dim=1).cuda().contiguous()
+    kv = kv.cuda()
+    odd = torch.empty(kv.numel() + 1, device="cuda")[1:].view(kv.shape)
+    odd.copy_(kv)
+    assert odd.data_ptr() % 16
+    outs = [ops.paged_attention(qkv, nh, nkv, d, pool, bt.cuda(), ctx, d ** -0.5, None) for pool in (kv, odd)]
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("nh,nkv,d,H", [(32, 4, 64, 256), (32, 8, 128, 512), (6, 2, 48, 96), (4, 4, 16, 64)])
 @pytest.mark.parametrize("q_lens,k_lens,window", [([1] * 20, [5, 17, 600, 64, 1, 129, 1023, 48, 300, 2, 33, 16, 700, 90, 250, 31, 32, 128, 257, 400], None),
                                                   ([1] * 64, [520] * 64, None), ([2, 1, 2] * 7, [300, 2, 129] * 7, None),
@@ -470,7 +486,7 @@ def padded_ctx(ops, k_lens, pad_to, nh, nkv, d):
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.int32)).cuda()
     small = plan["small"].reshape(-1, 4)
     ap = AttentionPlan(dev(small), None, dev(plan["splits"]), len(small), 0, plan["max_splits"],
-                       plan["num_small_tokens"], plan.get("long_context", False))
+                       plan["num_small_tokens"], plan.get("long_context", False), plan.get("even", False))
     cu = np.full(pad_to + 1, S, np.int32)
     cu[:S + 1] = np.arange(S + 1)
     klen = np.zeros(pad_to, np.int32)

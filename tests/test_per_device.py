@@ -102,11 +102,13 @@ def test_float32_product(lib, M):
     on_both_devices(lib, lambda: lib.pl_gemm_f32(P(4096), P(4096), P(4096), I(M), I(4096), I(2048), I(2048), I(2048), I(4096), P(0)))
 
 
+@pytest.mark.parametrize("kv", [4096, 4100])
 @pytest.mark.parametrize("d", [64, 128, 256])
-def test_float32_attention(lib, d):
+def test_float32_attention(lib, d, kv):
     from paged_llm_b200.kernels.ops import AttnParams
     p = AttnParams()
-    p.q = p.kv = p.out = p.block_table = p.cu_q = p.k_lens = p.work = 4096
+    p.q = p.out = p.block_table = p.cu_q = p.k_lens = p.work = 4096
+    p.kv = kv
     p.nh, p.nkv, p.d, p.ps, p.n_work, p.max_splits, p.num_pages = 4, 2, d, 16, 3, 1, 8
     on_both_devices(lib, lambda: lib.pl_attention_f32(ctypes.byref(p), P(0)))
 
