@@ -297,11 +297,14 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(AttnParams p, cons
     };
 
     if (own_here && warp == NW - 1) take(tc::saddr(own), hi, it.key_hi);       // while the first tile is still on its way
-    bool alive = true;
     for (int i = 0; i < count; ++i) {
         const int s = i % STAGES, key = tile_key(i);
-        alive = alive && tc::mbar_wait(&full[warp][s], (i / STAGES) & 1);
-        if (!__all_sync(0xffffffffu, alive)) break;         // (a copy that never arrived: counted, see kernel_timeouts)
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[warp][s], (i / STAGES) & 1))) {
+            // a copy that never arrived (counted, see kernel_timeouts): the others in flight must not land in what takes the
+            // ring's place
+            for (int j = i; j < asked; ++j) tc::mbar_wait(&full[warp][j % STAGES], (j / STAGES) & 1);
+            break;
+        }
         const uint32_t at = ring_at + s * S::TILE;
         if (key + KEYS > hi) {                              // the last tile: what lies behind the range must not be a NaN
             unsigned char* v = ring + (size_t)warp * STAGES * S::TILE + s * S::TILE + S::SIDE;

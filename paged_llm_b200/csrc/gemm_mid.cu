@@ -17,7 +17,7 @@
 // where s is 1, or, for X = h of an "add" product, the token's 1 / rms(x) from those sums: RMSNorm(x) * w = s * h, and a
 // factor per token can wait until after the product (h is rounded relative to its size either way).
 //
-// Every wait is bounded; a thread that gave up once stops waiting.
+// Every wait is bounded; a thread that gave up waits once more for the copies in flight and stops.
 //
 // Measured on a B200, us per product among others of its kind (graph of 16, cold weights), in brackets the library's
 // product with the kernel that then adds and norms, or multiplies by the activation, and the read of W at 6.45 TB/s:
@@ -159,7 +159,11 @@ __global__ void __launch_bounds__(MID_THREADS, 2) gemm_mid_kernel(MidParams p, c
             const uint32_t idesc = instr_desc(MID_ROWS, p.cols, false);
             for (int i = 0; i < steps; ++i) {
                 const int s = i % p.stages;
-                if (!mbar_wait(&full[s], (i / p.stages) & 1)) break;
+                if (!mbar_wait(&full[s], (i / p.stages) & 1)) {
+                    // the copies still in flight (none is asked for beyond these) must not land in what takes the ring's place
+                    for (int j = i; j < min(steps, i + p.stages); ++j) mbar_wait(&full[j % p.stages], (j / p.stages) & 1);
+                    break;
+                }
                 fence_after_sync();
                 const uint32_t wa = saddr(ring) + s * stage_bytes, xa = wa + MID_W_BYTES;
 #pragma unroll
