@@ -82,15 +82,9 @@ __device__ __forceinline__ void rotate_pair(uint4& lo, uint4& hi, const float2* 
     rotate_by(lo, hi, cs);
 }
 
-// Offset in elements of 16-byte chunk c of row r within that row.
-template <bool SWZ> __device__ __forceinline__ int attn_chunk(int r, int c) { return (SWZ ? c ^ (r & 7) : c) * 8; }
-
 template <int DPAD, int MW, int NW, int KPW, int STAGES = 2>
 struct AttnShape {
-    // Rows of 128 or 256 bytes lie as they are, their 16-byte chunks exchanged by the row's number (attn_chunk): no bank
-    // conflicts and no padding.
-    static constexpr bool SWZ = DPAD == 64 || DPAD == 128;
-    static constexpr int BM = 16 * MW, BN = KPW * NW, PITCH = SWZ ? DPAD : DPAD + 8, THREADS = 32 * MW * NW;
+    static constexpr int BM = 16 * MW, BN = KPW * NW, PITCH = DPAD + 8, THREADS = 32 * MW * NW;
     static constexpr int Q_BYTES = BM * PITCH * 2;                                // Q tile
     static constexpr int SMEM_BYTES = Q_BYTES + 2 * STAGES * BN * PITCH * 2;      // then K and V stages
     static constexpr int OWN_BYTES = 2 * KPW * PITCH * 2;                         // then (ROPE) a tile for one warp
@@ -272,7 +266,6 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
     using Shape = AttnShape<DPAD, MW, NW, KPW, STAGES>;
     constexpr int BM = Shape::BM, BN = Shape::BN, PITCH = Shape::PITCH, THREADS = Shape::THREADS;
     constexpr int CH = DPAD / 8;                          // 16-byte chunks per row
-    constexpr bool SWZ = Shape::SWZ;
     constexpr float LOG2E = 1.4426950408889634f;
     pdl_launch_dependents();
     // A block of a decode step waits for the kernel in front only after it has asked for its
@@ -352,7 +345,7 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
             const int po = p.ps_shift >= 0 ? key & (p.ps - 1) : key % p.ps;
             const bool ok = pg[i] >= 0;
             const __nv_bfloat16* src = ok ? kv_head + (size_t)pg[i] * page_stride + po * d : kv;
-            const int row = j0 + i * J_STEP, to = row * PITCH + attn_chunk<SWZ>(row, c8);
+            const int row = j0 + i * J_STEP, to = row * PITCH + c8 * 8;
             cp_async16(kd + to, src, ok ? 16 : 0);
             cp_async16(vd + to, ok ? src + v_off : kv, ok ? 16 : 0);
         }
@@ -410,9 +403,12 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
             else cp_async_commit();
         }
     }
-    // the pages of the tile that is asked for next are looked up an iteration earlier
-    int pages[LOAD_ITERS];
-    find_pages(pages, it.key_lo + (STAGES - 1) * BN);
+    // Prompt portions without modifiers look the pages of the next tile up an iteration earlier (300 and 500 tokens, 16 heads of
+    // 256: 105 -> 98 us).  A warp with a pipeline of its own has other warps to wait beside and no registers to spare
+    // for it (20 requests of 600 keys, 8 kv heads of 256: 84 -> 108 us), and the modified form spills.
+    constexpr bool AHEAD = !WP && !MOD;
+    int pages[AHEAD ? LOAD_ITERS : 1];
+    if constexpr (AHEAD) find_pages(pages, it.key_lo + (STAGES - 1) * BN);
     // (with ROPE) the angles of the first pairs this thread rotates: from a constant table
     const int hc = d / 16;                               // chunks per half of a head
     float4 angle[4];
@@ -449,12 +445,12 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
                 if (e != tid) rotate_pair(lo, hi, p.rope_table, p.rope_len, it.lk - it.nq + R / G, d, c8 * 8);
                 else if (rotate) rotate_by(lo, hi, angle);
             }
-            *reinterpret_cast<uint4*>(Qs + r * PITCH + attn_chunk<SWZ>(r, c8)) = lo;
-            *reinterpret_cast<uint4*>(Qs + r * PITCH + attn_chunk<SWZ>(r, hc + c8)) = hi;
+            *reinterpret_cast<uint4*>(Qs + r * PITCH + c8 * 8) = lo;
+            *reinterpret_cast<uint4*>(Qs + r * PITCH + d / 2 + c8 * 8) = hi;
         }
         const int padc = CH - 2 * hc;
         for (int e = tid; e < BM * padc; e += THREADS)
-            *reinterpret_cast<uint4*>(Qs + (e / padc) * PITCH + attn_chunk<SWZ>(e / padc, 2 * hc + e % padc)) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(Qs + (e / padc) * PITCH + d + (e % padc) * 8) = make_uint4(0, 0, 0, 0);
     } else {
         for (int e = tid; e < BM * CH; e += THREADS) {
             const int r = e / CH, c8 = e - r * CH;
@@ -462,7 +458,7 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
             uint4 v = make_uint4(0, 0, 0, 0);
             if (R < it.rows_total && c8 * 8 < d)
                 v = *reinterpret_cast<const uint4*>(q + (size_t)(it.q0 + R / G) * p.q_stride + (kvh * G + R % G) * d + c8 * 8);
-            *reinterpret_cast<uint4*>(Qs + r * PITCH + attn_chunk<SWZ>(r, c8)) = v;
+            *reinterpret_cast<uint4*>(Qs + r * PITCH + c8 * 8) = v;
         }
     }
     // (with ROPE) the step's own keys of this block's range as a tile of its own: rotated keys and values straight from the
@@ -496,24 +492,25 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
                     *reinterpret_cast<uint4*>(dst + v_off + d / 2) = vhi;
                 }
             }
-            const int at_lo = j * PITCH + attn_chunk<SWZ>(j, c8), at_hi = j * PITCH + attn_chunk<SWZ>(j, hc + c8);
+            const int at_lo = j * PITCH + c8 * 8, at_hi = j * PITCH + d / 2 + c8 * 8;
             *reinterpret_cast<uint4*>(Ko + at_lo) = klo;
             *reinterpret_cast<uint4*>(Ko + at_hi) = khi;
             *reinterpret_cast<uint4*>(Vo + at_lo) = vlo;
             *reinterpret_cast<uint4*>(Vo + at_hi) = vhi;
         }
         for (int e = tid; e < KPW * padc; e += THREADS) {
-            const int at = (e / padc) * PITCH + attn_chunk<SWZ>(e / padc, 2 * hc + e % padc);
+            const int at = (e / padc) * PITCH + d + (e % padc) * 8;
             *reinterpret_cast<uint4*>(Ko + at) = make_uint4(0, 0, 0, 0);
             *reinterpret_cast<uint4*>(Vo + at) = make_uint4(0, 0, 0, 0);
         }
     }
-    // the queries' fragments stay in registers where the tile is one row of warps and they are few
-    constexpr bool KEEP_Q = WP && DPAD <= 128;
+    // The queries' fragments stay in registers where the tile is one row of warps and they are few (64 requests, heads of 96:
+    // 41.8 -> 39.7 us; with modifiers there are none to spare: 40 requests, heads of 128, a cap: 41.5 -> 45.1).
+    constexpr bool KEEP_Q = WP && !MOD && DPAD <= 128;
     uint32_t qf[KEEP_Q ? DPAD / 16 : 1][4];
     auto load_q = [&](uint32_t (&a)[4], int kk) {
         const int r = wm * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-        ldmatrix_x4(a, Qs + r * PITCH + attn_chunk<SWZ>(lane, kk * 2 + (lane >> 4)));
+        ldmatrix_x4(a, Qs + r * PITCH + kk * 16 + (lane >> 4) * 8);
     };
     // scores, softmax and weighted values of the KPW keys from kbase on, which lie at kst and vst
     auto process_keys = [&](const __nv_bfloat16* kst, const __nv_bfloat16* vst, int kbase) {
@@ -544,7 +541,7 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
 #pragma unroll
                 for (int n2 = 0; n2 < KPW / 16; ++n2) {
                     uint32_t b[4];
-                    ldmatrix_x4(b, kst + (n2 * 16 + (lane & 7) + (lane >> 4) * 8) * PITCH + attn_chunk<SWZ>(lane, kk * 2 + ((lane >> 3) & 1)));
+                    ldmatrix_x4(b, kst + (n2 * 16 + (lane & 7) + (lane >> 4) * 8) * PITCH + kk * 16 + ((lane >> 3) & 1) * 8);
                     mma_bf16(sacc[2 * n2], a, b[0], b[1]);
                     mma_bf16(sacc[2 * n2 + 1], a, b[2], b[3]);
                 }
@@ -625,7 +622,7 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
 #pragma unroll
                 for (int d2 = 0; d2 < DPAD / 16; ++d2) {
                     uint32_t b[4];
-                    ldmatrix_x4_trans(b, vst + (k2 * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + attn_chunk<SWZ>(lane, d2 * 2 + (lane >> 4)));
+                    ldmatrix_x4_trans(b, vst + (k2 * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + d2 * 16 + (lane >> 4) * 8);
                     mma_bf16(oacc[2 * d2], pa[k2], b[0], b[1]);
                     mma_bf16(oacc[2 * d2 + 1], pa[k2], b[2], b[3]);
                 }
@@ -648,9 +645,13 @@ __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {
         // tile t + STAGES - 1 goes into the stage that tile t - 1 left (all warps are past it: the
         // barrier at the end of the iteration before); then all copies but those of the STAGES - 1
         // newest groups are awaited, which completes tile t (and the step's own keys)
-        if (t + STAGES - 1 < n_tiles) copy_tile(pages, (t + STAGES - 1) % STAGES, it.key_lo + (t + STAGES - 1) * BN);
-        else cp_async_commit();
-        find_pages(pages, it.key_lo + (t + STAGES) * BN);
+        if (t + STAGES - 1 < n_tiles) {
+            if constexpr (AHEAD) copy_tile(pages, (t + STAGES - 1) % STAGES, it.key_lo + (t + STAGES - 1) * BN);
+            else load_tile((t + STAGES - 1) % STAGES, it.key_lo + (t + STAGES - 1) * BN);
+        } else {
+            cp_async_commit();
+        }
+        if constexpr (AHEAD) find_pages(pages, it.key_lo + (t + STAGES) * BN);
         if (own_first) cp_async_wait<0>();
         else cp_async_wait<STAGES - 1>();
         if (WP) __syncwarp(); else __syncthreads();
@@ -795,7 +796,7 @@ PL_EXPORT int PL_CAT(pl_attention_bf16_d, PL_DPAD)(const AttnParams* params, cud
         // the score modifiers live in instantiations of their own of the mma.sync kernel (the tcgen05
         // kernels step aside for them)
         if (p.cluster > 0) return launch_attn_cluster<PL_DPAD, DEC_KPW, true, 2, DEC_NW, false, true>(p, stream);
-        if (p.is_small) return launch_attn_bf16<PL_DPAD, 1, DEC_NW, DEC_KPW, true, 2, true, true>(p, stream);
+        if (p.is_small) return launch_attn_bf16<PL_DPAD, 1, DEC_NW, DEC_KPW, true, 2, true>(p, stream);
         return launch_attn_bf16<PL_DPAD, PL_LARGE_MW, 1, 64, true>(p, stream);
     }
 #if PL_DPAD == 64 || PL_DPAD == 128
@@ -811,7 +812,11 @@ PL_EXPORT int PL_CAT(pl_attention_bf16_d, PL_DPAD)(const AttnParams* params, cud
         return launch_attn_bf16<PL_DPAD, 1, DEC_NW, DEC_KPW, false, 2, true, true, true>(p, stream);
     }
     if (p.cluster > 0) return launch_attn_cluster<PL_DPAD, DEC_KPW, false, 2, DEC_NW, false, true>(p, stream);
-    if (p.is_small) return launch_attn_bf16<PL_DPAD, 1, DEC_NW, DEC_KPW, false, 2, true, true>(p, stream);
+    // Starting early pays behind a kernel that lets this one start: the few-token product that rotates, in front of a step
+    // that only decodes (8 requests x 4,800 keys, 4 kv heads of 32: 19.4 -> 16.7 us).  The kernel that rotates in front
+    // of mixed steps does not.
+    if (p.is_small && p.small_rows > 0 && p.small_rows < 16) return launch_attn_bf16<PL_DPAD, 1, DEC_NW, DEC_KPW, false, 2, true, true>(p, stream);
+    if (p.is_small) return launch_attn_bf16<PL_DPAD, 1, DEC_NW, DEC_KPW, false, 2, true>(p, stream);
 #if PL_DPAD == 64 || PL_DPAD == 128
     // prefill tiles of head sizes 64 and 128 run on tcgen05 with tensor-memory accumulators
     static const bool no_tc = getenv("PAGED_LLM_B200_NO_TCGEN05") != nullptr;
