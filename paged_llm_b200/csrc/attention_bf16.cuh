@@ -247,16 +247,16 @@ __device__ __forceinline__ void attn_merge(const AttnParams& p, const AttnItem& 
 // MOD: the score modifiers of AttnParams (cap, bias by distance) are applied and the first keys may be kept beside a
 // window; the kernel without them is the one the Llama decoder runs and carries none of their code.
 // STAGES: key tiles in flight (a ring of that many K and V stages).
-// ROPE (cluster form only): q, k, v arrive as the projection left them.  The queries are rotated as
+// ROPE (decode forms only): q, k, v arrive as the projection left them.  The queries are rotated as
 // they are loaded (xiyiji/paged-llm llama.py:117-128: pairs i, i + d/2, float32 angles from the
 // table), the step's own keys are rotated, written to their page slots together with the values
-// (kv_cache.py:42-45) and taken from registers instead of from the cache: the separate kernel for
+// (kv_cache.py:42-45) and taken as a tile of their own instead of from the cache: the separate kernel for
 // rotary positions and the cache write is not needed.
 // WP (small shape only): every warp runs a copy pipeline of its own for the keys it multiplies, so
 // that the loop over key tiles has no block-wide barrier and the warps drift apart: one computes
 // while another waits for its keys.
-// EARLY (work list, small shape): as in the cluster form, the first keys are asked for before the wait for the kernel
-// in front.
+// EARLY (the cluster form, and the work list of steps that only decode): the first keys are asked for before the wait for
+// the kernel in front.
 template <int DPAD, int MW, int NW, int KPW, bool CLUSTER = false, bool MOD = false, int STAGES = 2, bool ROPE = false,
           bool WP = false, bool EARLY = CLUSTER>
 __global__ void __launch_bounds__(32 * MW * NW) attn_bf16_kernel(AttnParams p) {

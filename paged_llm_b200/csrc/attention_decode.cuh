@@ -400,7 +400,9 @@ int launch_shape(const AttnParams& p, cudaStream_t stream) {
 template <int D>
 int launch(const AttnParams& p, cudaStream_t stream) {
     PL_REQUIRE(p.rope_table == nullptr || p.rope_len > 0, "attention_decode: bad rotary table");
-    // Two blocks per SM in both shapes, by measurement (us per layer; attn_bf16_kernel, one range per request, before):
+    // Two blocks per SM in both shapes.  Three stages throughout: they win up to 4 us where blocks walk long ranges, two
+    // stages win up to 3 us where many blocks walk short ones (a rule by the plan's range length would have both; none is
+    // made).  Measured, us per layer; attn_bf16_kernel, one range per request, before:
     //                                                     before   here   two stages   the bytes at 6.45 TB/s
     //   64 requests x 641 keys, 4 kv heads of 64            14.4    9.8        11.0     6.5
     //   64 x 2,048                                          33.4   23.4        27.2    20.8

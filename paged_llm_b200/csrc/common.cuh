@@ -162,7 +162,6 @@ struct AttnParams {
     int nh, nkv, d, ps;
     int window;             // 0: none
     int is_small;           // items are (request, scratch base, split, splits), one tile per request
-                            // (2: the same, and the items' key ranges are long: see the dispatch of the kernels)
     float scale;
     int ps_shift;           // log2(ps) if ps is a power of two, else -1
     unsigned int* counters; // [requests * kv_heads] zeros, or null: the block of a request's kv head that
@@ -174,15 +173,15 @@ struct AttnParams {
     float softcap;          // > 0: s = softcap * tanh(s / softcap)
     const float* slopes;    // [nh] or null: s += slopes[head] * (key position - query position), a bias that grows
                             // with the distance to the key; applied after the cap
-    // Rotary positions inside the kernel (bfloat16 cluster form only; null: q, k, v are rotated and stored
-    // already).  `q` then is the projection's output [T, (nh + 2 nkv) d] (q heads, k heads, v heads): queries
+    // Rotary positions inside the kernel (bfloat16 decode steps only, as clusters or from a list of even ranges; null:
+    // q, k, v are rotated and stored already).  `q` then is the projection's output [T, (nh + 2 nkv) d] (q heads, k heads, v heads): queries
     // and the step's own keys are rotated over the whole head (pairs i, i + d/2) with the angles of this
     // table [rope_len, d/2] of (cos, sin), and the own keys and values are written to their page slots.
     const float2* rope_table;
     int rope_len;
     // A decode step padded to the size of its captured graph: rows [cu_q[pad_seqs], pad_to) of `out` belong to no
     // request (pad_seqs: the number of request slots, so cu_q[pad_seqs] is the number of real tokens, read on the
-    // device because a replayed graph sees other lengths).  The first block of the split-context kernels zeroes
+    // device because a replayed graph sees other lengths).  The first blocks of the split-context kernels zero
     // them, so that no fill kernel stands between two kernels of a layer.  pad_to == 0: nothing to do.
     int pad_seqs, pad_to;
     // Chunked mask: > 0: positions are cut into chunks of this many, counted from position 0 of the request, and a

@@ -1332,7 +1332,9 @@ class CudaOps:
             pad_tokens=pad_tokens, slots=self._attention_slots(head_dim), head_dim=head_dim)
 
     def _attention_slots(self, head_dim: int) -> int:
-        """Blocks of the decode kernel that are resident at a time, two per SM (0: its ranges are not cut evenly)."""
+        """Blocks of the decode kernel that are resident at a time, two per SM (0: its ranges are not cut evenly).  Two is right
+        for head sizes 64 and 128; the kernel of the others fits one to five, and gains by the even ranges all the same
+        (see `plan.BLOCK_KEYS`)."""
         if self.compute_dtype != torch.bfloat16 or not self.cluster_attention:
             return 0
         return 2 * self.num_sms
@@ -1391,7 +1393,7 @@ class CudaOps:
         softcap * tanh(score / softcap)) and `slopes` (a float32 tensor [nh]: head h adds
         slopes[h] * (key position - query position) to its scores) modify the scores; both off
         by default; `dist_bias` (float32 [nh, L]) adds dist_bias[h, min(query position - key position, L - 1)];
-        `chunk` c lets a query at position p see the keys from p - p % c on only.  `rope` (a prepared rotary encoding; only where the step runs as clusters, see
+        `chunk` c lets a query at position p see the keys from p - p % c on only.  `rope` (a prepared rotary encoding; only for a decode step, as clusters or in even ranges, see
         `qkv_attention`): qkv is the unrotated projection, and the kernel rotates q and the step's own
         keys and writes those keys and values to the cache itself.  `sink` (float32 [nh]): the softmax's denominator
         of head h also holds exp(sink[h]), a term without key or value that counts once however the keys are split.

@@ -38,7 +38,8 @@ def is_long_context(num_requests: int, num_kv_heads: int, num_sms: int, max_spli
     (at most `cluster_max` per request and kv head) would each walk more than `long_keys` keys.
     Such a step is split further, through the work list: about three blocks per SM, which is
     what is resident at a time and what it takes to keep memory busy with one block's latencies
-    (measured: 16 k context at batch 8, 2.05 ms per step as clusters of 5, 1.50 ms as 13 splits)."""
+    (measured on `attn_bf16_kernel`: 16 k context at batch 8, 2.05 ms per step as clusters of 5, 1.50 ms as 13 splits; the
+    line has not been measured again for the kernel that head sizes 64 and 128 run now)."""
     if cluster_max <= 0:
         return False
     cluster = min(wanted_splits(num_requests, num_kv_heads, num_sms, max_splits), cluster_max)
@@ -48,7 +49,10 @@ def is_long_context(num_requests: int, num_kv_heads: int, num_sms: int, max_spli
 
 
 # What a block costs beside its keys (its start, its query, the merge of its warps), and what the merge of the ranges of a
-# request adds, in keys: 4 and 1.2 us where a block reads some 85 keys per us.
+# request adds, in keys: 4 and 1.2 us where a block reads some 85 keys per us.  (Head size 64.  Other head sizes are planned
+# with the same figures and two blocks per SM, whatever kernel they run; against a cluster or one range per request, us per
+# layer: 20 requests of 300 to 3,500 keys, 8 kv heads of 16 30.1 -> 19.7, 8 of 32 35.7 -> 24.7, 8 of 96 73 -> 55, 8 of 256
+# 182 -> 158; 64 of 100 to 700, 8 of 96 53.9 -> 39.9.  A window of 512 gains from 40 requests on: 15.6 -> 16.2 at 20.)
 BLOCK_KEYS, MERGE_KEYS = 350, 100
 
 

@@ -79,8 +79,8 @@ def test_long_context_decode_steps_are_split_further():
                                              ([17] * 255 + [4000], 1, 256)])
 def test_even_ranges_cover_every_key_and_fit_the_graph(k_lens, nkv, pad):
     """Steps that are cut into even ranges: every request has all its ranges, the list fits the capacity that a captured
-    graph has, whatever the lengths, and its shape does not depend on them; a range is never shorter than an even share of
-    128 keys, so no block starts for a handful."""
+    graph has, whatever the lengths, and its shape does not depend on them; a request has no more ranges than its keys have
+    started multiples of 128 (129 keys may be cut into 96 and 33, since ranges begin at multiples of 32)."""
     kw = dict(cluster_max=8, long_keys=600, slots=296)
     S = len(k_lens)
     plan = general([1] * S, k_lens, 8, nkv, None, pad_requests=pad, fixed_capacity=True, **kw)
@@ -115,6 +115,8 @@ def test_even_ranges_do_not_depend_on_the_step_they_were_planned_for(k_lens, nkv
     """A replayed decode step keeps its plan until a context grows past another multiple of 128 keys.  So that it gives what
     the same step gives with a plan of its own, bit for bit, all lengths between two multiples have one plan."""
     kw = dict(cluster_max=8, long_keys=600, slots=296, pad_requests=pad, fixed_capacity=True)
+    from paged_llm_b200.kernels.ops import CudaOps
+    assert CudaOps.MIN_SPLIT_KEYS % planning.GRAIN == 0, "what a replayed step goes by"
     S = len(k_lens)
     first, last = [-(-k // 128) * 128 - 127 for k in k_lens], [-(-k // 128) * 128 for k in k_lens]
     plans = [general([1] * S, lens, 8, nkv, None, **kw) for lens in (k_lens, first, last)]
