@@ -763,6 +763,16 @@ PL_EXPORT int pl_attention_tc_timeouts() {
 #define PL_LARGE_MW (PL_DPAD <= 128 ? 8 : 4)
 PL_EXPORT int PL_CAT(pl_attention_bf16_rows_d, PL_DPAD)(int small) { return small ? 16 : 16 * PL_LARGE_MW; }
 
+#if PL_DPAD == 64 || PL_DPAD == 128
+// Whether plain prompt tiles over this pool run the kernel that can rotate their queries.
+PL_EXPORT int PL_CAT(pl_attention_bf16_rotates_d, PL_DPAD)(const void* kv, int num_pages, int nkv, int ps) {
+    static const bool off = getenv("PAGED_LLM_B200_NO_TCGEN05") != nullptr || getenv("PAGED_LLM_B200_TC_SERIAL") != nullptr;
+    int shift = 0;
+    while ((1 << shift) < ps) ++shift;
+    return !off && (1 << shift) == ps && tc2::takes_pool(kv, num_pages, nkv, ps, shift);
+}
+#endif
+
 PL_EXPORT int PL_CAT(pl_attention_bf16_d, PL_DPAD)(const AttnParams* params, cudaStream_t stream) {
     AttnParams p = *params;
     if (p.n_work == 0) return 0;
@@ -801,6 +811,11 @@ PL_EXPORT int PL_CAT(pl_attention_bf16_d, PL_DPAD)(const AttnParams* params, cud
     }
 #if PL_DPAD == 64 || PL_DPAD == 128
     if (dec::takes(p)) return dec::launch<PL_DPAD>(p, stream);
+    if (p.rope_table != nullptr && p.cluster <= 0 && !p.is_small) {
+        PL_REQUIRE(p.d == PL_DPAD && p.rope_len > 0 && PL_CAT(pl_attention_bf16_rotates_d, PL_DPAD)(p.kv, p.num_pages, p.nkv, p.ps),
+                   "attention_bf16: prompt tiles cannot rotate their queries here");
+        return tc2::launch<PL_DPAD>(p, stream);
+    }
 #endif
     // All forms of the small shape run warp-private copy pipelines (WP): 49 against 53 us at 64 requests x
     // 3,000 keys of head size 64, 110 against 115 at 8 x 16,384 of head size 128, no loss elsewhere.

@@ -498,7 +498,39 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     // Q tile: row R = token * G + head; eight 16-byte chunks per row and panel
-    for (int e = tid; e < BM * 8 * PANELS; e += THREADS) {
+    if (BIAS == 0 && p.rope_table != nullptr) {
+        // queries straight from the projection, rotated over the whole head: a chunk of the first half with its partner (of every
+        // query, one block loads it once, so that nothing is rotated twice)
+        constexpr int HC = D / 16, AT_ONCE = D == 64 ? 1 : 2;   // (pairs of chunks whose loads are in flight together: 1,224 against 1,284 us a prompt of 61 tokens with three)
+        for (int e0 = tid; e0 < BM * HC; e0 += AT_ONCE * THREADS) {
+            uint4 lo[AT_ONCE], hi[AT_ONCE];
+            float4 cs[AT_ONCE][4];
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const int e = e0 + u * THREADS, r = e / HC, c8 = e % HC, R = it.row_base + r;
+                lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) cs[u][k] = make_float4(1.f, 0.f, 1.f, 0.f);
+                if (e >= BM * HC || R >= it.rows_total) continue;
+                const __nv_bfloat16* src = q + (size_t)(it.q0 + R / G) * p.q_stride + (kvh * G + R % G) * D + c8 * 8;
+                lo[u] = *reinterpret_cast<const uint4*>(src);
+                hi[u] = *reinterpret_cast<const uint4*>(src + D / 2);
+                const int pos = it.lk - it.nq + R / G;
+                if (pos < 0 || pos >= p.rope_len) continue;
+                const float4* at = reinterpret_cast<const float4*>(p.rope_table + (size_t)pos * (D / 2) + c8 * 8);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) cs[u][k] = __ldg(at + k);
+            }
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const int e = e0 + u * THREADS, r = e / HC, c8 = e % HC, c2 = c8 + HC;
+                if (e >= BM * HC) continue;
+                rotate_by(lo[u], hi[u], cs[u]);
+                *reinterpret_cast<uint4*>(Qs + (c8 >> 3) * Q_PANEL + swz(r, c8 & 7)) = lo[u];
+                *reinterpret_cast<uint4*>(Qs + (c2 >> 3) * Q_PANEL + swz(r, c2 & 7)) = hi[u];
+            }
+        }
+    } else for (int e = tid; e < BM * 8 * PANELS; e += THREADS) {
         const int r = e / (8 * PANELS), c16 = e % (8 * PANELS);
         const int R = it.row_base + r;
         uint4 v = make_uint4(0, 0, 0, 0);
@@ -785,10 +817,10 @@ inline bool kv_tensor_map(CUtensorMap* out, const AttnParams& p) {
 
 // Whether this kernel takes the call: a page is a power of two of at least 8 tokens and the
 // pool's row numbers fit the 32-bit coordinates of a box.
-inline bool takes(const AttnParams& p) {
-    return p.ps_shift >= 3 && p.num_pages > 0 && (long long)p.num_pages * 2 * p.nkv * p.ps < (1ll << 31) &&
-           ((uintptr_t)p.kv & 15) == 0;
+inline bool takes_pool(const void* kv, int num_pages, int nkv, int ps, int ps_shift) {
+    return ps_shift >= 3 && num_pages > 0 && (long long)num_pages * 2 * nkv * ps < (1ll << 31) && ((uintptr_t)kv & 15) == 0;
 }
+inline bool takes(const AttnParams& p) { return takes_pool(p.kv, p.num_pages, p.nkv, p.ps, p.ps_shift); }
 
 template <int D, bool WIDE, int BIAS>
 inline int launch_as(const AttnParams& p, cudaStream_t stream) {

@@ -176,7 +176,8 @@ struct AttnParams {
     // Rotary positions inside the kernel (bfloat16 decode steps only, as clusters or from a list of even ranges; null:
     // q, k, v are rotated and stored already).  `q` then is the projection's output [T, (nh + 2 nkv) d] (q heads, k heads, v heads): queries
     // and the step's own keys are rotated over the whole head (pairs i, i + d/2) with the angles of this
-    // table [rope_len, d/2] of (cos, sin), and the own keys and values are written to their page slots.
+    // table [rope_len, d/2] of (cos, sin), and the own keys and values are written to their page slots.  For prompt tiles
+    // (neither clusters nor small items): the queries alone are not rotated yet.
     const float2* rope_table;
     int rope_len;
     // A decode step padded to the size of its captured graph: rows [cu_q[pad_seqs], pad_to) of `out` belong to no

@@ -1288,7 +1288,9 @@ class CudaOps:
         self.launches += 1
         return table
 
-    def rope_kv_write(self, qkv, nh, nkv, d, position, ctx, kv, block_table, write=True, value_from_key=False):
+    def rope_kv_write(self, qkv, nh, nkv, d, position, ctx, kv, block_table, write=True, value_from_key=False, rotated_later=0):
+        """Rotates the q and k columns of `qkv` in place and writes keys and values to their page slots.  `rotated_later` > 0: the
+        queries of requests that bring more than so many query rows per kv head are left as they are."""
         T = ctx.num_tokens
         assert qkv.is_contiguous() and qkv.shape[0] == T
         if position is not None:
@@ -1301,7 +1303,8 @@ class CudaOps:
         _check(self.core, self.core.pl_rope_kv_write(
             self._p(qkv), self._code(qkv), T, qkv.shape[1], self._p(table), table_len, rd, inter,
             self._p(ctx.positions), self._p(ctx.token_seq), self._p(block_table), block_table.shape[1],
-            self._p(kv), num_pages, nh, nkv, d, ps, 1 if write else 0, 1 if value_from_key else 0, self._stream))
+            self._p(kv), num_pages, nh, nkv, d, ps, 1 if write else 0, 1 if value_from_key else 0,
+            self._p(ctx.cu_seqlens_q if rotated_later else None), rotated_later, self._stream))
         self.launches += 1
 
     # ---- attention ---------------------------------------------------------------
@@ -1382,13 +1385,28 @@ class CudaOps:
         if inside:
             qkv = self.linear(h, w_qkv)
             return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, rope=position, chunk=chunk)
+        if (plan is not None and plan.n_large and write and softcap is None and slopes is None and position is not None
+                and not value_from_key and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens
+                and not self._skinny_ok(h, (nh + 2 * nkv) * d) and self._prompt_tiles_rotate(nh, nkv, d, kv, position)):
+            # the kernel of the prompt tiles rotates the queries it loads
+            qkv = self.linear(h, w_qkv)
+            self.rope_kv_write(qkv, nh, nkv, d, position, ctx, kv, block_table, rotated_later=self.SMALL_ROWS)
+            return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, chunk=chunk, tile_rope=position)
         qkv = self.qkv_rope_write(h, w_qkv, nh, nkv, d, position, ctx, kv, block_table, write=write,
                                   value_from_key=value_from_key)
         return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, softcap=softcap, slopes=slopes,
                                     chunk=chunk)
 
+    def _prompt_tiles_rotate(self, nh, nkv, d, kv, position) -> bool:
+        """Whether the kernel that prompt tiles of these heads run can rotate queries (the tcgen05 form by TMA)."""
+        if self.compute_dtype != torch.bfloat16 or kv.dtype != torch.bfloat16 or d not in (64, 128):
+            return False
+        lib, _ = self._attention_bf16(d)
+        return bool(position.table.is_contiguous() and wide(position.table)
+                    and getattr(lib, f"pl_attention_bf16_rotates_d{d}")(self._p(kv), kv.shape[0], nkv, kv.shape[3]))
+
     def paged_attention(self, qkv, nh, nkv, d, kv, block_table, ctx, scale, window, softcap=None, slopes=None,
-                        rope=None, chunk=None, dist_bias=None, sink=None, keep_first=0):
+                        rope=None, chunk=None, dist_bias=None, sink=None, keep_first=0, tile_rope=None):
         """Attention of the step's tokens over the paged cache.  `softcap` (scores become
         softcap * tanh(score / softcap)) and `slopes` (a float32 tensor [nh]: head h adds
         slopes[h] * (key position - query position) to its scores) modify the scores; both off
@@ -1397,7 +1415,8 @@ class CudaOps:
         `qkv_attention`): qkv is the unrotated projection, and the kernel rotates q and the step's own
         keys and writes those keys and values to the cache itself.  `sink` (float32 [nh]): the softmax's denominator
         of head h also holds exp(sink[h]), a term without key or value that counts once however the keys are split.
-        `keep_first` k (with a window): every query sees the request's first k keys too."""
+        `keep_first` k (with a window): every query sees the request's first k keys too.  `tile_rope` (a prepared rotary
+        encoding, see `qkv_attention`): the queries of prompt tiles are not rotated yet."""
         T = ctx.num_tokens
         keep_first = int(keep_first or 0) if window else 0
         plan = ctx.attention_plans[attention_plan_key(nh, nkv, window, d, chunk, keep_first)]
@@ -1476,6 +1495,8 @@ class CudaOps:
             p.scratch, p.scratch_floats, p.pad_to = 0, 0, 0
             p.work, p.n_work, p.is_small = plan.large.data_ptr(), plan.n_large, 0
             p.max_splits = 1
+            if tile_rope is not None:
+                p.rope_table, p.rope_len = tile_rope.table.data_ptr(), tile_rope.table.shape[0]
             _check(lib, fn(ctypes.byref(p), self._stream))
             self.launches += 1
         return out
