@@ -138,9 +138,9 @@ class CudaOps:
         self.mid_widths, self.mid_width_per_token, self.mid_features = (640, 4096), 20, 2 * self.num_sms * 128
         # Many tokens: this package's tcgen05 kernel (pairs of blocks on 256 x 256 tiles, fused epilogues) where it is at least
         # as fast as the library product followed by the elementwise kernel.  Measured: the gate/up product
-        # with SiLU-mul from 2,048 tokens on (77 us against 87 us, timed alone); the narrower products and fewer
-        # tokens are faster through the library.  PAGED_LLM_B200_GEMM_TC lists the kinds ("silu", "add", "plain", "all",
-        # "" for none) to run on it from 129 tokens on instead.
+        # with SiLU-mul from 2,048 tokens on (65 us against 80 us, timed alone), and below that where its tiles fill the machine
+        # (`_gate_up_tc_ok`); the narrower products are faster through the library.  PAGED_LLM_B200_GEMM_TC lists the
+        # kinds ("silu", "add", "plain", "all", "" for none) to run on it from 129 tokens on instead.
         tc_for = os.environ.get("PAGED_LLM_B200_GEMM_TC")
         self.gemm_tc_min_tokens = 2048 if tc_for is None else 129
         tc_for = "silu,moe" if tc_for is None else tc_for
@@ -502,6 +502,34 @@ class CudaOps:
                 and M >= self.gemm_tc_min_tokens
                 and K >= 64 and K % 64 == 0 and w.is_contiguous())
 
+    def _gate_up_tc_ok(self, h, w: torch.Tensor, I: int, activation: str) -> bool:
+        """Whether the tcgen05 kernel takes the gate/up product.  Below `gemm_tc_min_tokens` its tiles of 256 tokens and 128
+        features, a pair of SMs each, have to fill their waves: the products asked for are 0.75 of what the waves could do, 0.7
+        from the fourth wave on.  us, this kernel and the library's product with `act_mul`:
+
+            tokens    2,048 -> 5,632    2,048 -> 8,192    4,096 -> 14,336
+              256      18.4  15.7        19.7  21.0        57.6  60.7
+              384      27.3  19.1        28.5  26.3        92.6  79.1
+              512      27.4  25.2        28.6  32.1        96.4 107.4
+              576      28.0  27.6        38.3  35.3       120.4 104.8
+              768      28.3  30.9        40.0  45.2       124.5 151.0
+              832      37.7  35.1        50.0  54.9       163.8 167.0
+              960      37.9  36.2        51.3  56.7       189.0 190.1
+            1,024      37.9  43.9        51.9  57.4       185.9 224.6
+            1,408      50.3  57.7        73.6  82.0       249.2 294.8
+
+        (The line falls between the sides but for 2,048 -> 5,632 at 640 tokens and 2,048 -> 8,192 at 640, which it leaves to the
+        library: 28.3 against 30.3 and 38.9 against 43.9.  The tanh form of GELU has not been measured below 2,048.)"""
+        if self._gemm_tc_ok(h, w, "silu"):
+            return True
+        M, K = h.shape
+        if not ("silu" in self.gemm_tc_for and activation == "silu" and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+                and M > 64 and K >= 64 and K % 64 == 0 and w.is_contiguous() and wide(w) and wide(h)):
+            return False
+        pairs = self.num_sms // 2
+        waves = -(-(-(-M // 256) * -(-I // 128)) // pairs)
+        return M * I >= (0.75 if waves <= 3 else 0.7) * waves * pairs * 256 * 128
+
     def _gemm_tc(self, h: torch.Tensor, w: torch.Tensor, out, resid, N: int, epi: int) -> None:
         M, K = h.shape
         assert h.stride(1) == 1 and h.stride(0) % 8 == 0
@@ -609,7 +637,7 @@ class CudaOps:
             self.launches += 1
             return out
         h = self.materialize(h)
-        if self._gemm_tc_ok(h, w_gate_up, "silu") and h.is_contiguous() and I % 8 == 0:
+        if h.is_contiguous() and I % 8 == 0 and self._gate_up_tc_ok(h, w_gate_up, I, activation):
             out = torch.empty((M, I), dtype=torch.bfloat16, device=self.device)
             if activation == "silu":
                 self._gemm_tc(h, w_gate_up, out, None, I, 2)
