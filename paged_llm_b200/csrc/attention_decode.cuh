@@ -414,6 +414,19 @@ int launch(const AttnParams& p, cudaStream_t stream) {
     //   1 x 641, 4 kv heads of 64                            5.5    5.6         5.4     0.1
     // Head size 64 with four warps of four stages: 11.0 at the first, 22.5 at the third; eight warps of four stages
     // (one block per SM): 14.7 and 34.
+    //
+    // Steps of so many requests that blocks come and go: with two stages three blocks fit an SM (80 registers: up to eight
+    // query rows), and the list is cut for as many (CudaOps._three_blocks says when).  Requests x kv heads, with contexts of
+    // 16 to 400, 300, 300 to 1,200 and 1,200 keys, three stages / two:
+    //    93 x 8     13.9 10.7   16.2 12.5   28.7 24.7   41.4 37.8
+    //   186 x 4     14.5 11.1   16.5 12.8   29.1 25.4   42.0 38.3
+    // and of 40 to 160, 70 to 777, 500, 200 to 1,400 and 1,500:
+    //   256 x 4     17.1 13.3   28.0 23.7   31.7 27.1   40.5 37.8    64.3  64.2
+    //   256 x 8     30.6 23.0   51.6 42.2   54.9 46.1   73.3 67.3   119.7 117.3
+    if constexpr (D == 64) {
+        if (p.three_blocks && p.cluster <= 0 && p.small_rows > 0 && p.small_rows <= 8)
+            return p.rope_table != nullptr ? launch_as<D, 1, 8, 2, false, true>(p, stream) : launch_as<D, 1, 8, 2, false, false>(p, stream);
+    }
     if constexpr (D == 64) return launch_shape<D, 8, 3>(p, stream);
     else return launch_shape<D, 4, 3>(p, stream);
 }

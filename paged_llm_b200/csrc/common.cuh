@@ -202,6 +202,8 @@ struct AttnParams {
     int keep_first;
     // Small items: no request brings more query rows per kv head than this (0: up to 16).
     int small_rows;
+    // The list was cut for three blocks per SM (see dec::launch).
+    int three_blocks;
 };
 
 // What the sink adds to a row's sum of exponentials taken relative to the maximum `m` (natural-log units; -inf:

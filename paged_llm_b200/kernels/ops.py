@@ -49,7 +49,7 @@ class AttnParams(ctypes.Structure):
         ("scale", c_float), ("ps_shift", c_int), ("counters", c_void_p), ("num_pages", c_int), ("cluster", c_int),
         ("softcap", c_float), ("slopes", c_void_p), ("rope_table", c_void_p), ("rope_len", c_int),
         ("pad_seqs", c_int), ("pad_to", c_int), ("chunk", c_int), ("dist_bias", c_void_p), ("dist_len", c_int),
-        ("sink", c_void_p), ("keep_first", c_int), ("small_rows", c_int),
+        ("sink", c_void_p), ("keep_first", c_int), ("small_rows", c_int), ("three_blocks", c_int),
     ]
 
 
@@ -1355,12 +1355,24 @@ class CudaOps:
 
     def plan_attention(self, q_lens, k_lens, group_size, num_kv_heads, window, head_dim, chunk=None, keep_first=None,
                        pad_requests=None, fixed_capacity=False, pad_tokens=None) -> dict:
+        slots = self._attention_slots(head_dim)
+        if slots and not window and not chunk and pad_tokens is None and max(q_lens, default=0) == 1 and self._three_blocks(
+                pad_requests if fixed_capacity else len(q_lens), num_kv_heads, group_size, head_dim):
+            slots = 3 * self.num_sms
         return planning.plan_attention(
             q_lens, k_lens, group_size, num_kv_heads, window, chunk=chunk, keep_first=keep_first, small_rows=self.SMALL_ROWS,
             large_rows=self._large_rows(head_dim), min_split_keys=self.MIN_SPLIT_KEYS, num_sms=self.num_sms,
             max_splits=self.MAX_SPLITS, pad_requests=pad_requests, fixed_capacity=fixed_capacity,
             cluster_max=self.MAX_CLUSTER if self.cluster_attention else 0, long_keys=self.CLUSTER_KEYS,
-            pad_tokens=pad_tokens, slots=self._attention_slots(head_dim), head_dim=head_dim)
+            pad_tokens=pad_tokens, slots=slots, head_dim=head_dim)
+
+    def _three_blocks(self, num_requests: int, num_kv_heads: int, group_size: int, head_dim: int) -> bool:
+        """Whether a decode step of so many requests runs the decode kernel's form of which three blocks fit an SM (times at
+        dec::launch): with more than six (request, kv head) pairs per SM, of which a step padded to the size of its graph may use
+        two thirds to three quarters.  With fewer it still wins 5 to 25 % where contexts are short or differ, but where they are
+        long and alike the last, nearly empty round of blocks with the shorter ring takes longer (130 requests of 4 kv heads, 600
+        keys 14.9 -> 14.3 us, but 1,200 keys 28.4 -> 33.2)."""
+        return bool(head_dim == 64 and group_size <= 8 and num_requests * num_kv_heads > 6 * self.num_sms)
 
     def _attention_slots(self, head_dim: int) -> int:
         """Blocks of the decode kernel that are resident at a time, two per SM (0: its ranges are not cut evenly).  Two is right
@@ -1466,6 +1478,8 @@ class CudaOps:
         # (a step of mixed items may replay a graph in which later steps bring more tokens per small item)
         p.small_rows = nh // nkv if max(ctx.host.q_lens) == 1 and not plan.n_large else self.SMALL_ROWS
         p.window, p.scale, p.max_splits = int(window or 0), float(scale), plan.max_splits
+        p.three_blocks = int(plan.even and not plan.n_large and max(ctx.host.q_lens) == 1 and not window and not chunk
+                             and self._three_blocks(ctx.num_seqs, nkv, nh // nkv, d))
         p.softcap = float(softcap or 0.0)
         p.chunk, p.keep_first = int(chunk or 0), keep_first
         if slopes is not None:
