@@ -1579,28 +1579,31 @@ class CudaOps:
         if self._sample_dev is None or self._sample_dev.numel() < words:
             self._sample_keep.append(self._sample_dev)              # a kernel in flight may still read the old one
             self._sample_dev = torch.empty(max(2 * words, 1024), dtype=torch.int64, device=dev)
-            self._sample_ring = [[torch.empty(max(2 * words, 1024), dtype=torch.int64, pin_memory=True), None]
-                                 for _ in range(4)]
+            # (buffer, the same as 8-byte and as 4-byte words, event of its last copy, whether that was recorded)
+            self._sample_ring = []
+            for _ in range(4):
+                buf = torch.empty(max(2 * words, 1024), dtype=torch.int64, pin_memory=True)
+                self._sample_ring.append([buf, buf.numpy().view(np.uint64), buf.numpy().view(np.float32), torch.cuda.Event(), False])
         slot = self._sample_ring[self._sample_pos % len(self._sample_ring)]
         self._sample_pos += 1
-        if slot[1] is not None:
-            slot[1].synchronize()                                   # its last copy has left the buffer
-        host = slot[0].numpy()
-        host[:rows] = np.ascontiguousarray(seeds, np.uint64).view(np.int64)
-        host[rows:2 * rows] = np.ascontiguousarray(counters, np.uint64).view(np.int64)
-        tail = host[2 * rows:words].view(np.float32)
-        tail[:rows] = temps
-        tail[rows:2 * rows] = top_p
-        tail[2 * rows:3 * rows].view(np.int32)[:] = top_k
-        self.copy_h2d(self._sample_dev, slot[0], words * 8)
-        slot[1] = torch.cuda.Event()
-        slot[1].record()
-        s, c = self._sample_dev[:rows], self._sample_dev[rows:2 * rows]
-        tail_dev = self._sample_dev[2 * rows:words].view(torch.float32)
-        t, pp, k = tail_dev[:rows], tail_dev[rows:2 * rows], tail_dev[2 * rows:3 * rows].view(torch.int32)
+        buf, wide_words, floats, event, used = slot
+        if used:
+            event.synchronize()                                     # its last copy has left the buffer
+        wide_words[:rows] = seeds
+        wide_words[rows:2 * rows] = counters
+        at = 4 * rows                                               # (in 4-byte words)
+        floats[at:at + rows] = temps
+        floats[at + rows:at + 2 * rows] = top_p
+        floats[at + 2 * rows:at + 3 * rows].view(np.int32)[:] = top_k
+        stream = self._stream
+        base = self._sample_dev.data_ptr()
+        _check(self.core, self.core.pl_copy_h2d(c_void_p(base), self._p(buf), c_longlong(words * 8), stream))
+        event.record()
+        slot[4] = True
         out = torch.empty(rows, dtype=torch.int32, device=dev)
-        _check(self.core, self.core.pl_sample(self._p(logits), self._p(out), rows, V, c_longlong(logits.stride(0)),
-                                              self._p(t), self._p(k), self._p(pp), self._p(s), self._p(c),
-                                              self._stream))
+        tail = base + 16 * rows
+        _check(self.core, self.core.pl_sample(self._p(logits), self._p(out), rows, V, c_longlong(logits.stride(0)), c_void_p(tail),
+                                              c_void_p(tail + 8 * rows), c_void_p(tail + 4 * rows), c_void_p(base),
+                                              c_void_p(base + 8 * rows), stream))
         self.launches += 1
         return out
