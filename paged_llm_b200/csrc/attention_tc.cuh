@@ -443,10 +443,14 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
     using SH = Shape<D>;
     constexpr int PANELS = SH::PANELS, STAGES = SH::STAGES, Q_PANEL = SH::Q_PANEL, K_PANEL = SH::K_PANEL;
     constexpr int Q_BYTES = SH::Q_BYTES, K_BYTES = SH::K_BYTES;
+    // The list, the lengths and the block tables are older than the step: a block finds its item, sets its barriers up and takes
+    // its tensor memory before it waits for the kernel in front.
     pdl_launch_dependents();
-    pdl_wait();
     const AttnItem it = attn_decode_item(p, blockIdx.x / p.nkv, BM, BN);
-    if (!it.valid) return;
+    if (!it.valid) {
+        pdl_wait();                                            // (a grid is only done once the kernel in front is)
+        return;
+    }
 
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
@@ -497,6 +501,8 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
             for (int b = 0; b < SH::BIAS_SLOTS; ++b) mbar_init(&b_full[b], 64);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    pdl_wait();
+    asm volatile("fence.proxy.async;\n" ::: "memory");         // keys and values that the kernel in front wrote by ordinary stores
     // Q tile: row R = token * G + head; eight 16-byte chunks per row and panel
     if (BIAS == 0 && p.rope_table != nullptr) {
         // queries straight from the projection, rotated over the whole head: a chunk of the first half with its partner (of every
