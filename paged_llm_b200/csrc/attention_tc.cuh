@@ -283,13 +283,14 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_kernel(AttnParams p) {
 }
 
 inline int launch(const AttnParams& p, cudaStream_t stream) {
-    static bool attr_set = false;
-    if (!attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        PL_CUDA(cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared));
-        attr_set = true;
-    }
+    static PerDevice<char> ready;
+    if (!ready.get("attention_tc", [](char&) {
+            PL_CUDA(cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+            PL_CUDA(cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared));
+            return 0;
+        }))
+        return 1;
     PL_CUDA(launch_pdl(attn_tc_kernel, dim3(p.n_work * p.nkv), dim3(THREADS), (size_t)SMEM_BYTES, stream, p));
     return 0;
 }
@@ -835,15 +836,16 @@ inline bool takes(const AttnParams& p) { return takes_pool(p.kv, p.num_pages, p.
 
 template <int D, bool WIDE, int BIAS>
 inline int launch_as(const AttnParams& p, cudaStream_t stream) {
-    static bool attr_set = false;
+    static PerDevice<char> ready;
     auto kernel = attn_tc2_kernel<D, WIDE, BIAS>;
     constexpr int smem = BIAS == 2 ? Shape<D>::SMEM_BIAS : Shape<D>::SMEM_BYTES;
-    if (!attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared));
-        attr_set = true;
-    }
+    if (!ready.get("attention_tc", [&](char&) {
+            PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared));
+            return 0;
+        }))
+        return 1;
     alignas(64) CUtensorMap map;
     if (!kv_tensor_map(&map, p)) return 1;
     PL_CUDA(launch_pdl(kernel, dim3(p.n_work * p.nkv), dim3(THREADS), (size_t)smem, stream, p, map));

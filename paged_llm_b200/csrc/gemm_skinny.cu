@@ -538,23 +538,20 @@ __global__ void __launch_bounds__(SK_THREADS, 1) gemm_skinny_kernel(SkinnyParams
     }
 }
 
-int g_num_sms = 0;
-
 template <int EPI, int NT, bool NORM, int XC>
 int launch_skinny(const SkinnyParams& p, cudaStream_t stream) {
     constexpr size_t smem = (size_t)SK_STAGES * SK_STAGE_BYTES + (size_t)2 * SK_CONSUMERS * NT * 128 * sizeof(float) +
                             (16 + 256) * sizeof(float) + 2 * SK_STAGES * sizeof(uint64_t);
-    static bool attr_set = false;
-    if (!attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(gemm_skinny_kernel<EPI, NT, NORM, XC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
-    if (g_num_sms == 0) {
+    static PerDevice<int> found;
+    const int* sms = found.get("gemm_skinny", [](int& n) {
         int dev = 0;
         PL_CUDA(cudaGetDevice(&dev));
-        PL_CUDA(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
-    }
-    const int grid = p.num_blocks < g_num_sms ? p.num_blocks : g_num_sms;
+        PL_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+        PL_CUDA(cudaFuncSetAttribute(gemm_skinny_kernel<EPI, NT, NORM, XC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return 0;
+    });
+    if (!sms) return 1;
+    const int grid = p.num_blocks < *sms ? p.num_blocks : *sms;
     PL_CUDA(launch_pdl(gemm_skinny_kernel<EPI, NT, NORM, XC>, dim3(grid), dim3(SK_THREADS), smem, stream, p));
     return 0;
 }

@@ -211,13 +211,15 @@ int gemm_tc_duo_launch(const void* X, int ldx, const void* W, void* Y, int ldy, 
     PL_REQUIRE(epi == TC_ADD ? (resid != nullptr && N % 4 == 0 && ((uintptr_t)resid & 15) == 0)
                              : (Y != nullptr && ldy >= N && ((uintptr_t)Y & 15) == 0),
                "gemm_tc_duo: output missing, misaligned or ldy < N");
-    static int sms = 0;
-    if (sms == 0) {
+    static PerDevice<int> found;
+    const int* sms = found.get("gemm_tc_duo", [](int& n) {
         int dev = 0;
         PL_CUDA(cudaGetDevice(&dev));
-        PL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        PL_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
         PL_CUDA(cudaFuncSetAttribute(gemm_tc_duo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DUO_SMEM));
-    }
+        return 0;
+    });
+    if (!sms) return 1;
     TcParams p = {};
     p.Y = Y;
     p.resid = resid;
@@ -240,7 +242,7 @@ int gemm_tc_duo_launch(const void* X, int ldx, const void* W, void* Y, int ldy, 
         !tensor_map_bf16(&w_map, W, (unsigned long long)w_rows, (unsigned long long)K, (unsigned long long)K, 128))
         return 1;
     const int pairs = p.m_tiles / 2 * p.n_tiles;
-    const int max_pairs = sms / 2;
+    const int max_pairs = *sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((pairs < max_pairs ? pairs : max_pairs) * 2);
     cfg.blockDim = dim3(TC_THREADS);

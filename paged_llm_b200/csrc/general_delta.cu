@@ -314,11 +314,12 @@ int launch_gd_step_as(const GdIn& in, const GdTail& tail, float* state, long lon
                       void* out, cudaStream_t stream) {
     const int vec = in.d % 4 == 0 && state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
     constexpr int smem = gs_smem(NPER * GS_LANES);
-    static bool opted = false;
-    if (!opted) {
-        PL_CUDA(cudaFuncSetAttribute(gd_step_kernel<T, NPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        opted = true;
-    }
+    static PerDevice<char> ready;
+    if (!ready.get("general_delta_step", [](char&) {
+            PL_CUDA(cudaFuncSetAttribute(gd_step_kernel<T, NPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            return 0;
+        }))
+        return 1;
     PL_CUDA(launch_pdl(gd_step_kernel<T, NPER>, dim3((unsigned)num_seqs * in.H), dim3(GS_THREADS), (size_t)smem, stream, in, tail, state,
                        state_stride, cu_q, slots, (T*)out, vec));
     return 0;
@@ -657,13 +658,14 @@ __global__ void __launch_bounds__(GC_THREADS) gd_chunk_scan_kernel(int H, int d,
 template <typename T, int DP>
 int launch_gd_chunks(const GdIn& in, const float* z, float* buf, int slots_of_chunks, float* state, long long state_stride, const int* cu_q,
                      const int* slots, int num_seqs, float* out, cudaStream_t stream) {
-    static bool opted = false;
-    if (!opted) {
-        PL_CUDA(cudaFuncSetAttribute(gd_chunk_prepare_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, gc_prepare_smem(DP)));
-        PL_CUDA(cudaFuncSetAttribute(gd_chunk_prepare_kernel<T, DP>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-        PL_CUDA(cudaFuncSetAttribute(gd_chunk_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, gc_scan_smem(DP)));
-        opted = true;
-    }
+    static PerDevice<char> ready;
+    if (!ready.get("general_delta_chunks", [](char&) {
+            PL_CUDA(cudaFuncSetAttribute(gd_chunk_prepare_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, gc_prepare_smem(DP)));
+            PL_CUDA(cudaFuncSetAttribute(gd_chunk_prepare_kernel<T, DP>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+            PL_CUDA(cudaFuncSetAttribute(gd_chunk_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, gc_scan_smem(DP)));
+            return 0;
+        }))
+        return 1;
     PL_REQUIRE(in.H <= 65535, "general_delta: %d heads", in.H);
     gd_chunk_prepare_kernel<T, DP><<<dim3(slots_of_chunks, in.H), GC_THREADS, gc_prepare_smem(DP), stream>>>(in, z, cu_q, slots, num_seqs, buf);
     PL_LAUNCHED("general_delta_chunk_prepare");

@@ -691,11 +691,12 @@ PL_EXPORT int pl_delta_rule(float* u, int C, const void* proj, int dtype, int ld
         const dim3 grid(num_seqs, H, (dv + cols - 1) / cols);                                                                  \
         PL_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "delta_rule: %d heads of %d values", H, dv);                            \
         const size_t smem = (size_t)2 * dr_stage_floats((N) * (L), cols) * sizeof(float);                                      \
-        static bool opted = false;                                                                                             \
-        if (!opted && smem > 48 * 1024) {                                                                                      \
-            PL_CUDA(cudaFuncSetAttribute(delta_scan_kernel<N, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));    \
-            opted = true;                                                                                                      \
-        }                                                                                                                      \
+        static PerDevice<char> ready;                                                                                          \
+        if (smem > 48 * 1024 && !ready.get("delta_scan", [&](char&) {                                                          \
+                PL_CUDA(cudaFuncSetAttribute(delta_scan_kernel<N, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+                return 0;                                                                                                      \
+            }))                                                                                                                \
+            return 1;                                                                                                          \
         delta_scan_kernel<N, L><<<grid, DR_THREADS, smem, stream>>>(u, C, bg, H, G, d, dv, state, state_stride, state_off,     \
                                                                     cu_q, slots, out, vec);                                    \
     } while (0)

@@ -525,12 +525,15 @@ PL_EXPORT int pl_sample(const float* logits, int* out, int rows, int V, long lon
                         const unsigned long long* counters, cudaStream_t stream) {
     if (rows == 0) return 0;
     PL_REQUIRE(rows > 0 && V > 0 && V < (1 << 21) && row_stride >= V, "sample: bad sizes rows=%d V=%d", rows, V);
-    static int sms = 0;
-    if (sms == 0) {
+    static PerDevice<int> found;
+    const int* at = found.get("sample", [](int& n) {
         int dev = 0;
         PL_CUDA(cudaGetDevice(&dev));
-        PL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
+        PL_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+        return 0;
+    });
+    if (!at) return 1;
+    const int sms = *at;
     // Few rows of a large vocabulary: a cluster of blocks per row, as large as still gives every block an SM of its own
     // (measured at 128,256 tokens with top-p: 8 rows 238 -> 58 us with clusters of 8; 64 rows are best with 2).
     const size_t rs = (size_t)row_stride;

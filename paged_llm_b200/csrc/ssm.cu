@@ -500,11 +500,12 @@ static int launch_scan4(const float* xbc, int C, int inner, int G, int N, int H,
     constexpr int COLS = 512 / LPG;
     const size_t smem = (size_t)2 * (2 * SCAN_TOK * LPG * NV * 4 + SCAN_TOK * COLS + 2 * SCAN_TOK) * sizeof(float);
     auto kernel = ssm_scan4_kernel<LPG, NV>;
-    static bool attr_set = false;
-    if (smem > 48 * 1024 && !attr_set) {
-        PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static PerDevice<char> ready;
+    if (smem > 48 * 1024 && !ready.get("ssm_scan", [&](char&) {
+            PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            return 0;
+        }))
+        return 1;
     kernel<<<dim3(num_seqs, H, (P + COLS - 1) / COLS), 128, smem, stream>>>(xbc, C, inner, G, N, H, P, dt, decay, Dskip, state,
                                                                            state_stride, ssm_off, cu_q, slots, y);
     PL_LAUNCHED("ssm_scan");
@@ -544,11 +545,12 @@ PL_EXPORT int pl_ssm_scan(const float* xbc, int C, int inner, int G, int N, int 
     do {                                                                                                                   \
         const size_t smem = (size_t)2 * (2 * SCAN_TOK * L * NP + SCAN_TOK * (128 / L) + 2 * SCAN_TOK) * sizeof(float);     \
         auto kernel = ssm_scan_kernel<NP, V, L>;                                                                           \
-        static bool attr_set = false;                                                                                      \
-        if (smem > 48 * 1024 && !attr_set) {                                                                               \
-            PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                 \
-            attr_set = true;                                                                                               \
-        }                                                                                                                  \
+        static PerDevice<char> ready;                                                                                      \
+        if (smem > 48 * 1024 && !ready.get("ssm_scan", [&](char&) {                                                        \
+                PL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));             \
+                return 0;                                                                                                  \
+            }))                                                                                                            \
+            return 1;                                                                                                      \
         kernel<<<grid, 128, smem, stream>>>(xbc, C, inner, G, N, H, P, dt, decay, Dskip, state, state_stride, ssm_off, cu_q, \
                                             slots, y);                                                                     \
     } while (0)
