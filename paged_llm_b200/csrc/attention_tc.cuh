@@ -38,7 +38,6 @@ constexpr int TMEM_COLS = 256;           // S: columns 0..127, O: 128..191
 constexpr int Q_BYTES = BM * 128, KV_STAGE_BYTES = BN * 128, P_BYTES = BM * BN * 2;
 constexpr int SMEM_BYTES = Q_BYTES + 3 * KV_STAGE_BYTES + P_BYTES + 1024;     // + alignment slack
 __global__ void __launch_bounds__(THREADS, 2) attn_tc_kernel(AttnParams p) {
-    pdl_launch_dependents();
     pdl_wait();
     const AttnItem it = attn_decode_item(p, blockIdx.x / p.nkv, BM, BN);
     if (!it.valid) return;
@@ -63,6 +62,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc_kernel(AttnParams p) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(&tmem_base_slot)),
                      "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+        pdl_launch_dependents();                               // (not before: see attn_tc2_kernel)
     }
     if (tid == 0) {
         mbar_init(&bar_s, 1);
@@ -444,14 +444,11 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
     using SH = Shape<D>;
     constexpr int PANELS = SH::PANELS, STAGES = SH::STAGES, Q_PANEL = SH::Q_PANEL, K_PANEL = SH::K_PANEL;
     constexpr int Q_BYTES = SH::Q_BYTES, K_BYTES = SH::K_BYTES;
-    // The list, the lengths and the block tables are older than the step: a block finds its item, sets its barriers up and takes
-    // its tensor memory before it waits for the kernel in front.
-    pdl_launch_dependents();
+    // (Finding the item, setting the barriers up and taking tensor memory ahead of this wait gained nothing in whole steps, and
+    // holds tensor memory that a library product in front may still ask for.)
+    pdl_wait();
     const AttnItem it = attn_decode_item(p, blockIdx.x / p.nkv, BM, BN);
-    if (!it.valid) {
-        pdl_wait();                                            // (a grid is only done once the kernel in front is)
-        return;
-    }
+    if (!it.valid) return;
 
     extern __shared__ unsigned char smem_unaligned[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_unaligned + 1023) & ~(uintptr_t)1023);
@@ -485,6 +482,9 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(&tmem_base_slot)),
                      "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+        // The kernel behind may only come now: one that took tensor memory before its own wait, while a block here has still to
+        // get its columns, would wait for this grid and this grid for it.
+        pdl_launch_dependents();
     }
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -502,7 +502,6 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
             for (int b = 0; b < SH::BIAS_SLOTS; ++b) mbar_init(&b_full[b], 64);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    pdl_wait();
     asm volatile("fence.proxy.async;\n" ::: "memory");         // keys and values that the kernel in front wrote by ordinary stores
     // Q tile: row R = token * G + head; eight 16-byte chunks per row and panel
     if (BIAS == 0 && p.rope_table != nullptr) {
