@@ -148,7 +148,8 @@ class CudaOps:
         # (token, expert) pairs of a step from which the routed experts' products take the grouped tcgen05 form
         self.moe_tc_min_pairs = 2048
         self.cluster_attention = os.environ.get("PAGED_LLM_B200_NO_CLUSTER") is None   # decode attention as clusters
-        # decode steps of more than 16 tokens: rotary positions and the cache write inside the attention kernel
+        # steps of more than 16 tokens: rotary positions and the cache write of decode steps, and the rotation of the queries of
+        # prompt tiles, inside the attention kernel
         self.rope_in_attention = os.environ.get("PAGED_LLM_B200_NO_ROPE_IN_ATTENTION") is None
         # lanes that share a column of the delta rule's state (8 unless 16 or 32 is asked for, for measurements)
         self.delta_lanes = int(os.environ.get("PAGED_LLM_B200_DELTA_LANES", "0"))
@@ -1410,9 +1411,9 @@ class CudaOps:
                       softcap=None, slopes=None, chunk=None, value_from_key=False) -> torch.Tensor:
         """The mixer's whole front: fused q/k/v projection, rotary positions on q and k, k and v written
         to the cache, attention over the pages.  Returns [T, nh * d].  It is `qkv_rope_write` followed by
-        `paged_attention`, but for a decode step of more than 16 tokens (the projection's epilogue does
-        not rotate then) rotation and cache write happen inside the attention kernel instead of in
-        a kernel of their own."""
+        `paged_attention`, but for a step of more than 16 tokens (the projection's epilogue does not rotate
+        then) the attention takes a part of that over, unless `rope_in_attention` is off: in a decode step
+        rotation and cache write, in a step with prompt tiles the rotation of their queries."""
         M = h.shape[0]
         plan = ctx.attention_plans.get(attention_plan_key(nh, nkv, window, d, chunk))
         inside = (plan is not None and write and softcap is None and slopes is None and position is not None
@@ -1425,8 +1426,9 @@ class CudaOps:
         if inside:
             qkv = self.linear(h, w_qkv)
             return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, rope=position, chunk=chunk)
-        if (plan is not None and plan.n_large and write and softcap is None and slopes is None and position is not None
-                and not value_from_key and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens
+        if (self.rope_in_attention and plan is not None and plan.n_large and write and softcap is None and slopes is None
+                and position is not None and not value_from_key
+                and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens
                 and not self._skinny_ok(h, (nh + 2 * nkv) * d) and self._prompt_tiles_rotate(nh, nkv, d, kv, position)):
             # the kernel of the prompt tiles rotates the queries it loads
             qkv = self.linear(h, w_qkv)
