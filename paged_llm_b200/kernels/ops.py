@@ -1579,7 +1579,9 @@ class CudaOps:
         # values.
         words = 2 * rows + (3 * rows + 1) // 2
         if self._sample_dev is None or self._sample_dev.numel() < words:
-            self._sample_keep.append(self._sample_dev)              # a kernel in flight may still read the old one
+            # a kernel in flight may still read the old one, and copies the old ring (they were issued by address: the pool of
+            # pinned memory would hand buffers that nobody holds out again at once)
+            self._sample_keep.append((self._sample_dev, self._sample_ring))
             self._sample_dev = torch.empty(max(2 * words, 1024), dtype=torch.int64, device=dev)
             # (buffer, the same as 8-byte and as 4-byte words, event of its last copy, whether that was recorded)
             self._sample_ring = []

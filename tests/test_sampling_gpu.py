@@ -95,3 +95,29 @@ def test_draws_are_those_of_the_filter(ops, rows, kind, top_k, top_p):
     if kind == "masked":
         row[1000:] = -math.inf
     check(ops, row, 0.7, top_k, top_p, rows)
+
+
+def test_more_rows_while_copies_are_in_flight():
+    """A draw whose parameters are still to be copied, behind a long kernel, when a draw of more rows takes larger buffers: what
+    the pool of pinned memory hands out next must not be the buffer that the copy reads."""
+    from paged_llm_b200.kernels.ops import CudaOps
+    ops, rows, V = CudaOps("cuda"), 8, 1000
+    g = torch.Generator(device="cuda").manual_seed(5)
+    logits = torch.empty(400, V, device="cuda").normal_(0.0, 0.3, generator=g)
+    args = lambda n: (np.full(n, 1.0, np.float32), np.zeros(n, np.int32), np.full(n, 1.0, np.float32),
+                      np.arange(n, dtype=np.uint64) + np.uint64(77), np.full(n, 9, np.uint64))
+    want = CudaOps("cuda").sample(logits[:rows], *args(rows)).tolist()
+    # (what is allocated behind the long kernel comes from the pools: an allocation by the driver might wait for it)
+    spare = [torch.empty(n, dtype=torch.int64, pin_memory=True) for n in [1024] * 16 + [2800] * 4]
+    spare.append(torch.empty(1 << 18, device="cuda"))
+    del spare
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)                                  # some 0.1 s
+    got = ops.sample(logits[:rows], *args(rows))
+    many = ops.sample(logits, *args(400))
+    taken = [torch.zeros(1024, dtype=torch.int64, pin_memory=True) for _ in range(32)]
+    for t in taken:                                                 # (parameters of eight rows too, with another seed)
+        t[:2 * rows] = 123456789
+        t.view(torch.float32)[4 * rows:6 * rows] = 1.0
+    torch.cuda.synchronize()
+    assert got.tolist() == want and many[:rows].tolist() == want and len(taken) == 32
