@@ -311,7 +311,7 @@ inline int launch(const AttnParams& p, cudaStream_t stream) {
 //   k_full[s], v_full[s]    the boxes of a stage of keys / values have landed (TMA complete_tx)
 //   k_empty[s], v_empty[s]  the product reading the stage is done              (tcgen05.commit)
 //   s_full[b]    S[b] = Q K^T is in tensor memory        (tcgen05.commit)
-//   p_full[b]    P[b] is in tensor memory, O is rescaled, stray value rows are zeroed (softmax threads)
+//   p_full[b]    P[b] is in tensor memory, O is rescaled, stray value rows are zeroed (an arrival per softmax warp)
 //   pv_done[b]   O += P[b] V is done: S[b] may be written again (tcgen05.commit)
 // The product warp issues P(t) V(t) and then S(t+2), while the softmax warps work on S(t+1).
 // Key tiles start at multiples of 64 so that a box never straddles a page; keys outside the
@@ -435,6 +435,19 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
     for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Eight elements of the first half of a query and their partners, rotated as rope_kv_write_kernel does (two (cos, sin) per float4).
+__device__ __forceinline__ void rotate_chunk(uint4& lo, uint4& hi, const float4 (&cs)[4]) {
+    __nv_bfloat162* a = reinterpret_cast<__nv_bfloat162*>(&lo);
+    __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&hi);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 t = cs[k];
+        const float2 x = __bfloat1622float2(a[k]), y = __bfloat1622float2(b[k]);
+        a[k] = __floats2bfloat162_rn(rotated_lo(x.x, y.x, t.x, t.y), rotated_lo(x.y, y.y, t.z, t.w));
+        b[k] = __floats2bfloat162_rn(rotated_hi(x.x, y.x, t.x, t.y), rotated_hi(x.y, y.y, t.z, t.w));
+    }
+}
+
 // WIDE (head size 128 only): O += P V as one product 128 x 128 x 16 per step, the value panels
 // being the two 64-column groups of its MN-major operand, instead of one product per panel.
 // BIAS: 0 neither a bias by distance nor kept first keys (the kernel of plain prompts carries none of their code), 1 a bias,
@@ -507,22 +520,25 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
     if (BIAS == 0 && p.rope_table != nullptr) {
         // queries straight from the projection, rotated over the whole head: a chunk of the first half with its partner (of every
         // query, one block loads it once, so that nothing is rotated twice)
-        constexpr int HC = D / 16, AT_ONCE = D == 64 ? 1 : 2;   // (pairs of chunks whose loads are in flight together: 1,224 against 1,284 us a prompt of 61 tokens with three)
+        // AT_ONCE: pairs of chunks whose loads are in flight together (head size 64: 1,224 us for a prompt of 61 tokens, 1,284 with
+        // three; 128, whose threads have twice the chunks, has been timed with two alone)
+        constexpr int HC = D / 16, AT_ONCE = D == 64 ? 1 : 2;
         for (int e0 = tid; e0 < BM * HC; e0 += AT_ONCE * THREADS) {
             uint4 lo[AT_ONCE], hi[AT_ONCE];
             float4 cs[AT_ONCE][4];
+            bool turns[AT_ONCE];
 #pragma unroll
             for (int u = 0; u < AT_ONCE; ++u) {
                 const int e = e0 + u * THREADS, r = e / HC, c8 = e % HC, R = it.row_base + r;
                 lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) cs[u][k] = make_float4(1.f, 0.f, 1.f, 0.f);
+                turns[u] = false;
                 if (e >= BM * HC || R >= it.rows_total) continue;
                 const __nv_bfloat16* src = q + (size_t)(it.q0 + R / G) * p.q_stride + (kvh * G + R % G) * D + c8 * 8;
                 lo[u] = *reinterpret_cast<const uint4*>(src);
                 hi[u] = *reinterpret_cast<const uint4*>(src + D / 2);
                 const int pos = it.lk - it.nq + R / G;
                 if (pos < 0 || pos >= p.rope_len) continue;
+                turns[u] = true;
                 const float4* at = reinterpret_cast<const float4*>(p.rope_table + (size_t)pos * (D / 2) + c8 * 8);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) cs[u][k] = __ldg(at + k);
@@ -531,7 +547,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_tc2_kernel(AttnParams p, cons
             for (int u = 0; u < AT_ONCE; ++u) {
                 const int e = e0 + u * THREADS, r = e / HC, c8 = e % HC, c2 = c8 + HC;
                 if (e >= BM * HC) continue;
-                rotate_by(lo[u], hi[u], cs[u]);
+                if (turns[u]) rotate_chunk(lo[u], hi[u], cs[u]);
                 *reinterpret_cast<uint4*>(Qs + (c8 >> 3) * Q_PANEL + swz(r, c8 & 7)) = lo[u];
                 *reinterpret_cast<uint4*>(Qs + (c2 >> 3) * Q_PANEL + swz(r, c2 & 7)) = hi[u];
             }

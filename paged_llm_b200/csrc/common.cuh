@@ -64,6 +64,12 @@ template <typename T> class PerDevice {
     }
 };
 
+// The pair (x, y) rotated by (cos, sin): x cos - y sin and y cos + x sin, each with its second product rounded by itself.
+// Spelled out because the compiler may fuse either product with the sum, and does so differently from kernel to kernel: what is
+// rotated by the kernel that writes the cache or by the attention has to come out the same to the bit.
+__device__ __forceinline__ float rotated_lo(float x, float y, float c, float s) { return __fmaf_rn(x, c, -__fmul_rn(y, s)); }
+__device__ __forceinline__ float rotated_hi(float x, float y, float c, float s) { return __fmaf_rn(y, c, __fmul_rn(x, s)); }
+
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <typename T> __device__ __forceinline__ T from_float(float v);

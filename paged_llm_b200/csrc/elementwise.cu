@@ -391,10 +391,10 @@ __global__ void rope_kv_write_kernel(T* __restrict__ qkv, int row_stride, const 
                 const float4 a = Vec4<T>::load(head + j), b = Vec4<T>::load(head + j + half);
                 const float4 c01 = *reinterpret_cast<const float4*>(cs + j);
                 const float4 c23 = *reinterpret_cast<const float4*>(cs + j + 2);
-                const float4 lo = make_float4(a.x * c01.x - b.x * c01.y, a.y * c01.z - b.y * c01.w,
-                                              a.z * c23.x - b.z * c23.y, a.w * c23.z - b.w * c23.w);
-                const float4 hi = make_float4(b.x * c01.x + a.x * c01.y, b.y * c01.z + a.y * c01.w,
-                                              b.z * c23.x + a.z * c23.y, b.w * c23.z + a.w * c23.w);
+                const float4 lo = make_float4(rotated_lo(a.x, b.x, c01.x, c01.y), rotated_lo(a.y, b.y, c01.z, c01.w),
+                                              rotated_lo(a.z, b.z, c23.x, c23.y), rotated_lo(a.w, b.w, c23.z, c23.w));
+                const float4 hi = make_float4(rotated_hi(a.x, b.x, c01.x, c01.y), rotated_hi(a.y, b.y, c01.z, c01.w),
+                                              rotated_hi(a.z, b.z, c23.x, c23.y), rotated_hi(a.w, b.w, c23.z, c23.w));
                 Vec4<T>::store(head + j, lo);
                 Vec4<T>::store(head + j + half, hi);
                 if (h >= nh && to_cache) {
