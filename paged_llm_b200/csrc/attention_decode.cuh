@@ -400,9 +400,8 @@ int launch_shape(const AttnParams& p, cudaStream_t stream) {
 template <int D>
 int launch(const AttnParams& p, cudaStream_t stream) {
     PL_REQUIRE(p.rope_table == nullptr || p.rope_len > 0, "attention_decode: bad rotary table");
-    // Two blocks per SM in both shapes.  Three stages throughout: they win up to 4 us where blocks walk long ranges, two
-    // stages win up to 3 us where many blocks walk short ones (a rule by the plan's range length would have both; none is
-    // made).  Measured, us per layer; attn_bf16_kernel, one range per request, before:
+    // Two blocks per SM of three stages in both shapes, but for steps of very many requests (below): three stages win up to 4 us
+    // where blocks walk long ranges, two win up to 3 us where many blocks walk short ones.  Measured, us per layer; attn_bf16_kernel, one range per request, before:
     //                                                     before   here   two stages   the bytes at 6.45 TB/s
     //   64 requests x 641 keys, 4 kv heads of 64            14.4    9.8        11.0     6.5
     //   64 x 2,048                                          33.4   23.4        27.2    20.8
@@ -416,13 +415,21 @@ int launch(const AttnParams& p, cudaStream_t stream) {
     // (one block per SM): 14.7 and 34.
     //
     // Steps of so many requests that blocks come and go: with two stages three blocks fit an SM (80 registers: up to eight
-    // query rows), and the list is cut for as many (CudaOps._three_blocks says when).  Requests x kv heads, with contexts of
-    // 16 to 400, 300, 300 to 1,200 and 1,200 keys, three stages / two:
-    //    93 x 8     13.9 10.7   16.2 12.5   28.7 24.7   41.4 37.8
-    //   186 x 4     14.5 11.1   16.5 12.8   29.1 25.4   42.0 38.3
-    // and of 40 to 160, 70 to 777, 500, 200 to 1,400 and 1,500:
-    //   256 x 4     17.1 13.3   28.0 23.7   31.7 27.1   40.5 37.8    64.3  64.2
-    //   256 x 8     30.6 23.0   51.6 42.2   54.9 46.1   73.3 67.3   119.7 117.3
+    // query rows), and the list is cut for as many (CudaOps._three_blocks says when).  us per layer, three stages / two, with
+    // contexts all of one length, and from a quarter of it to seven quarters:
+    //                             100          500         1,200        2,000         3,000         4,000
+    //   112 x 8     alike      17.9  15.0   32.0  27.6   52.6  52.1   80.4  78.9   113.2 112.1   144.9 143.9
+    //               mixed      18.2  15.4   30.5  27.1   53.0  48.9   78.3  73.2   108.5 104.4   140.6 137.0
+    //   192 x 8     alike      26.6  21.0   48.6  41.0   82.2  78.1  124.9 120.8   179.7 174.1   234.0 228.8
+    //               mixed      28.2  22.3   49.5  42.7   85.5  79.4  125.9 120.3   178.7 173.6   230.9 225.3
+    //   256 x 4     alike      19.5  16.3   35.9  31.7   59.2  58.1   87.5  86.0   123.4 122.4   159.2 159.2
+    //               mixed      20.5  17.4   36.9  32.3   60.9  56.8   88.1  83.4   123.4 119.2   157.7 154.1
+    //    33 x 32    alike      19.1  15.9   35.8  31.7   59.9  57.8   87.3  86.3   121.6 123.1   159.0 159.5
+    // Fewer pairs in a graph of as many (the rest of its requests are empty):
+    //    97 x 8     alike      14.6  11.8   28.9  23.8   45.1  43.5   67.6  64.5    94.7  92.2   120.8 119.3
+    //               mixed      16.1  13.2   27.9  23.6   45.0  41.0   66.1  63.0    91.6  90.6   119.3 120.3
+    // A tenth of the requests with six times the keys of the others, 8 kv heads, longest context 4,800: 112 50.2 49.7, 192 80.9
+    // 75.8; longest 16,000: 97 122.4 124.9, 112 140.8 142.3, 192 230.8 230.8.
     if constexpr (D == 64) {
         if (p.three_blocks && p.cluster <= 0 && p.small_rows > 0 && p.small_rows <= 8)
             return p.rope_table != nullptr ? launch_as<D, 1, 8, 2, false, true>(p, stream) : launch_as<D, 1, 8, 2, false, false>(p, stream);

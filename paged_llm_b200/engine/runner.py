@@ -356,12 +356,15 @@ class ModelRunner:
                 return None
             bucket = next(b for b in self.GRAPH_BUCKETS if b >= len(items))
             # few requests with long contexts take other attention kernels than the same batch
-            # with short ones: a graph of its own
+            # with short ones, and so do very many requests: a graph of its own
             # (and since the plan keys of a model may differ in kv heads, the class is kept per key)
             classify = getattr(self.ops, "long_context_class", None)
+            beyond = getattr(self.ops, "beyond_three_blocks", None)
             if classify is not None and self.plan_keys:
                 longest = max(it.seq.num_computed_tokens for it in items) + 1
-                classes = tuple(bool(not key[2] and not any(key[4:]) and classify(bucket, key[1], longest))
+                classes = tuple(bool(not key[2] and not any(key[4:])
+                                     and (classify(bucket, key[1], longest)
+                                          or beyond is not None and beyond(bucket, key[1], key[0], key[3], longest)))
                                 for key in self.plan_keys)
                 if any(classes):
                     return ("decode", bucket, classes)

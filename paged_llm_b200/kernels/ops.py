@@ -1358,7 +1358,7 @@ class CudaOps:
                        pad_requests=None, fixed_capacity=False, pad_tokens=None) -> dict:
         slots = self._attention_slots(head_dim)
         if slots and not window and not chunk and pad_tokens is None and max(q_lens, default=0) == 1 and self._three_blocks(
-                pad_requests if fixed_capacity else len(q_lens), num_kv_heads, group_size, head_dim):
+                pad_requests if fixed_capacity else len(q_lens), num_kv_heads, group_size, head_dim, max(k_lens)):
             slots = 3 * self.num_sms
         return planning.plan_attention(
             q_lens, k_lens, group_size, num_kv_heads, window, chunk=chunk, keep_first=keep_first, small_rows=self.SMALL_ROWS,
@@ -1367,17 +1367,28 @@ class CudaOps:
             cluster_max=self.MAX_CLUSTER if self.cluster_attention else 0, long_keys=self.CLUSTER_KEYS,
             pad_tokens=pad_tokens, slots=slots, head_dim=head_dim)
 
-    def _three_blocks(self, num_requests: int, num_kv_heads: int, group_size: int, head_dim: int) -> bool:
-        """Whether a decode step of so many requests runs the decode kernel's form of which three blocks fit an SM (times at
-        dec::launch): with more than six (request, kv head) pairs per SM, of which a step padded to the size of its graph may use
-        two thirds to three quarters.  With fewer it still wins 5 to 25 % where contexts are short or differ, but where they are
-        long and alike the last, nearly empty round of blocks with the shorter ring takes longer (130 requests of 4 kv heads, 600
-        keys 14.9 -> 14.3 us, but 1,200 keys 28.4 -> 33.2)."""
-        return bool(head_dim == 64 and group_size <= 8 and num_requests * num_kv_heads > 6 * self.num_sms)
+    THREE_BLOCKS_KEYS = 4096
+
+    def _three_blocks(self, num_requests: int, num_kv_heads: int, group_size: int, head_dim: int, longest: int = 1) -> bool:
+        """Whether a decode step of so many requests, the longest context of `longest` keys, runs the decode kernel's form of
+        which three blocks fit an SM (times at dec::launch): with more than six (request, kv head) pairs per SM, of which a step
+        padded to the size of its graph may use two thirds to three quarters.  With fewer it still wins 5 to 25 % where contexts
+        are short or differ, but where they are long and alike the last, nearly empty round of blocks with the shorter ring takes
+        longer (131 requests of 4 kv heads, 500 keys 20.3 -> 19.6 us, but 1,200 keys 33.4 -> 36.5).  With longer contexts the
+        gain is used up and the shorter ring loses up to 3 % (97 requests of 8 kv heads, 1,500 to 10,500 keys 172.1 -> 176.6);
+        up to 4,096 keys no step measured lost more than 1 %."""
+        return bool(head_dim == 64 and group_size <= 8 and num_requests * num_kv_heads > 6 * self.num_sms
+                    and longest <= self.THREE_BLOCKS_KEYS)
+
+    def beyond_three_blocks(self, num_requests: int, num_kv_heads: int, group_size: int, head_dim: int, longest: int) -> bool:
+        """True if a decode step has requests enough for that form and a context too long for it: like the long-context class,
+        a graph of its own."""
+        return bool(self._attention_slots(head_dim) and longest > self.THREE_BLOCKS_KEYS
+                    and self._three_blocks(num_requests, num_kv_heads, group_size, head_dim))
 
     def _attention_slots(self, head_dim: int) -> int:
         """Blocks of the decode kernel that are resident at a time, two per SM (0: its ranges are not cut evenly).  Two is right
-        for head sizes 64 and 128; the kernel of the others fits one to five, and gains by the even ranges all the same
+        for head sizes 64 (but see `_three_blocks`) and 128; the kernel of the others fits one to five, and gains by the even ranges all the same
         (see `plan.BLOCK_KEYS`)."""
         if self.compute_dtype != torch.bfloat16 or not self.cluster_attention:
             return 0
@@ -1481,7 +1492,8 @@ class CudaOps:
         p.small_rows = nh // nkv if max(ctx.host.q_lens) == 1 and not plan.n_large else self.SMALL_ROWS
         p.window, p.scale, p.max_splits = int(window or 0), float(scale), plan.max_splits
         p.three_blocks = int(plan.even and not plan.n_large and max(ctx.host.q_lens) == 1 and not window and not chunk
-                             and self._three_blocks(ctx.num_seqs, nkv, nh // nkv, d))
+                             and self._three_blocks(ctx.num_seqs, nkv, nh // nkv, d)             # (few steps look further)
+                             and self._three_blocks(ctx.num_seqs, nkv, nh // nkv, d, max(ctx.host.starts) + 1))
         p.softcap = float(softcap or 0.0)
         p.chunk, p.keep_first = int(chunk or 0), keep_first
         if slopes is not None:

@@ -45,12 +45,54 @@ def test_many_requests(ops, nh, nkv, n, lens, inside):
     assert ctx.attention_plans[(nh // nkv, nkv, None, d)].even
     kv_dev, old = kv.cuda(), ops.rope_in_attention
     ops.rope_in_attention = inside
+    lib, attention = ops._attention_bf16(d)
+    asked = []
+
+    def noting(p, stream):
+        asked.append((p._obj.three_blocks, p._obj.small_rows, bool(p._obj.rope_table)))
+        return attention(p, stream)
+
+    ops._attention_bf16 = lambda _: (lib, noting)
     try:
         out = ops.qkv_attention(h, w, nh, nkv, d, rope, ctx, kv_dev, bt.cuda(), d ** -0.5, None).float().cpu()
     finally:
         ops.rope_in_attention = old
+        del ops._attention_bf16
+    assert asked == [(1, nh // nkv, inside)]                                  # what dec::launch takes that form by
     for s, L in enumerate(k_lens):
         qs = torch.zeros(L, nh, d)
         qs[L - 1] = q_rot[s]
         want = plain_llama.causal_attention(qs, keys[s], vals[s], d ** -0.5, window=None)[L - 1:].reshape(1, nh * d)
         torch.testing.assert_close(out[s:s + 1], want, atol=tol(dtype), rtol=tol(dtype), msg=f"request {s}")
+
+
+def test_contexts_that_grow_past_the_form(tmp_path):
+    """64 requests of 16 kv heads: short contexts take the form, and a graph of their own takes over once the longest context is
+    past the limit (lowered here).  Logits on both sides, replayed and launched one by one, against the float32 engine's."""
+    from paged_llm_b200.engine.replay import TraceReplayer
+    from tests import schedules
+    from tests.helpers import assert_bf16_close_to_f32, requests_for
+    from tests.tiny import make_folder
+    hf = {"architectures": ["LlamaForCausalLM"], "vocab_size": 256, "hidden_size": 128, "intermediate_size": 256, "num_hidden_layers": 2,
+          "num_attention_heads": 16, "num_key_value_heads": 16, "head_dim": 64, "rms_norm_eps": 1e-5, "rope_theta": 10000.0,
+          "max_position_embeddings": 512, "tie_word_embeddings": False, "hidden_act": "silu", "torch_dtype": "float32"}
+    folder = make_folder(tmp_path, hf, dict(seed=4, std=0.05, norm_std=0.1))
+    reqs = requests_for(256, [21 + i % 5 for i in range(60)] + [45] * 4, seed=9)
+    steps = [{"step": 0, "entries": [{"id": r, "tokens": t[:-6], "want": []} for r, t in reqs.items()], "end": []}]
+    for i in range(6):
+        steps.append({"step": i + 1, "entries": [{"id": r, "tokens": [t[len(t) - 6 + i]], "want": [0]} for r, t in reqs.items()],
+                      "end": list(reqs) if i == 5 else []})
+
+    def logits(dtype, **kw):
+        rp = TraceReplayer(folder, dtype, 64 * 64, **kw)
+        rp.ops.THREE_BLOCKS_KEYS = 42                              # the longest context is 40 to 45 keys
+        return schedules.collect(steps, {rec["step"]: rp.step(rec) for rec in steps}), rp
+
+    want, _ = logits("float32")
+    launched, rp = logits("bfloat16", enforce_eager=True)
+    assert rp.runner.num_graph_steps == 0
+    replayed, rp = logits("bfloat16")
+    assert {("decode", 64), ("decode", 64, (True,))} <= set(rp.runner._graphs) and rp.runner.num_graph_steps == 6
+    for rid in reqs:
+        assert_bf16_close_to_f32(launched[rid], want[rid], f"launched {rid}")
+        assert_bf16_close_to_f32(replayed[rid], want[rid], f"replayed {rid}")
