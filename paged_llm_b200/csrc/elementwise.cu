@@ -355,14 +355,22 @@ PL_EXPORT int pl_rope_table(const float* inv_freq, float* table, int P, int half
 // v_from_k: the row has no value columns; the values are the keys as projected, before the rotation.
 // cu_q non-null: the q heads of requests with more than q_rows query rows per kv head are left alone: the attention rotates
 // them as it loads them (a prompt of 2,048 tokens, 32 + 2 x 4 heads of 64: 8.9 us with all heads, four fifths of it q).
+// early: this kernel starts ahead of the end of the one in front, and lets the one behind it do so.  Worth it in front of the
+// tensor-core attention of head sizes 64 and 128 in bfloat16; other attention kernels lose, since their waiting blocks take the
+// places of blocks that have work.  us for projection (512 -> 6,144 at most), rotation and attention, without / with:
+//   bfloat16, prompt of 512 tokens: 32 + 2 x 8 heads of 16 18.7 27.4, of 32 21.8 26.9, of 80 44.3 43.3; of 128, capped scores 32.7 32.3
+//   bfloat16, 33 decoding requests beside two portions of 64: heads of 16 34.6 39.2, of 32 41.5 49.1, of 80 96.3 101.9, of 128,
+//     capped scores 105.5 113.2; of 64 40.2 39.7, of 128 66.8 65.3
+//   bfloat16, 24 portions of 4 tokens: heads of 64 26.4 25.1, of 128 34.1 30.5
+//   float32, heads of 64: prompt of 61 tokens 43.5 47.9, 33 decoding requests beside two portions 255 275
 template <typename T>
 __global__ void rope_kv_write_kernel(T* __restrict__ qkv, int row_stride, const float2* __restrict__ table,
                                      int table_len, int rotary_dim, int interleaved, const int* __restrict__ positions,
                                      const int* __restrict__ token_seq, const int* __restrict__ block_table,
                                      int bt_stride, T* __restrict__ kv, int num_pages, int nh, int nkv, int d, int ps,
-                                     int write, int vec, int v_from_k, const int* __restrict__ cu_q, int q_rows) {
+                                     int write, int vec, int v_from_k, const int* __restrict__ cu_q, int q_rows, int early) {
     const int t = blockIdx.x;
-    pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
     pdl_wait();
     const int s = token_seq[t];
     if (s < 0) return;
@@ -484,7 +492,7 @@ __global__ void rope_kv_write_kernel(T* __restrict__ qkv, int row_stride, const 
 PL_EXPORT int pl_rope_kv_write(void* qkv, int dtype, int T, int row_stride, const float* table, int table_len,
                                int rotary_dim, int interleaved, const int* positions, const int* token_seq,
                                const int* block_table, int bt_stride, void* kv, int num_pages, int nh, int nkv, int d,
-                               int ps, int write, int v_from_k, const int* cu_q, int q_rows, cudaStream_t stream) {
+                               int ps, int write, int v_from_k, const int* cu_q, int q_rows, int early, cudaStream_t stream) {
     if (T == 0) return 0;
     PL_REQUIRE(T > 0 && nh > 0 && nkv > 0 && d > 0 && ps > 0, "rope_kv_write: bad sizes");
     PL_REQUIRE(rotary_dim >= 0 && rotary_dim <= d && rotary_dim % 2 == 0, "rope_kv_write: rotary_dim=%d with d=%d",
@@ -495,16 +503,24 @@ PL_EXPORT int pl_rope_kv_write(void* qkv, int dtype, int T, int row_stride, cons
     // 16-byte path: heads, halves and rows start on 16-byte boundaries
     const int vec = d % per16 == 0 && row_stride % per16 == 0 && (rotary_dim / 2) % per16 == 0 &&
                     (((uintptr_t)qkv | (uintptr_t)kv | (uintptr_t)table) & 15) == 0;
-    if (dtype == PL_F32)
-        PL_CUDA(launch_pdl(rope_kv_write_kernel<float>, dim3(T), dim3(threads), 0, stream, (float*)qkv, row_stride, (const float2*)table,
-                           table_len, rotary_dim, interleaved, positions, token_seq, block_table, bt_stride, (float*)kv, num_pages,
-                           nh, nkv, d, ps, write, vec, v_from_k, cu_q, q_rows));
-    else if (dtype == PL_BF16)
-        PL_CUDA(launch_pdl(rope_kv_write_kernel<__nv_bfloat16>, dim3(T), dim3(threads), 0, stream, (__nv_bfloat16*)qkv, row_stride,
-                           (const float2*)table, table_len, rotary_dim, interleaved, positions, token_seq, block_table, bt_stride,
-                           (__nv_bfloat16*)kv, num_pages, nh, nkv, d, ps, write, vec, v_from_k, cu_q, q_rows));
-    else
-        return pl_fail("rope_kv_write: unknown dtype %d", dtype);
+#define PL_ROPE(TT)                                                                                                            \
+    do {                                                                                                                       \
+        if (early) {                                                                                                           \
+            PL_CUDA(launch_pdl(rope_kv_write_kernel<TT>, dim3(T), dim3(threads), 0, stream, (TT*)qkv, row_stride,              \
+                               (const float2*)table, table_len, rotary_dim, interleaved, positions, token_seq, block_table,    \
+                               bt_stride, (TT*)kv, num_pages, nh, nkv, d, ps, write, vec, v_from_k, cu_q, q_rows, early));     \
+        } else {                                                                                                               \
+            rope_kv_write_kernel<TT><<<T, threads, 0, stream>>>((TT*)qkv, row_stride, (const float2*)table, table_len,         \
+                                                                rotary_dim, interleaved, positions, token_seq, block_table,    \
+                                                                bt_stride, (TT*)kv, num_pages, nh, nkv, d, ps, write, vec,     \
+                                                                v_from_k, cu_q, q_rows, early);                                \
+            PL_LAUNCHED("rope_kv_write");                                                                                      \
+        }                                                                                                                      \
+    } while (0)
+    if (dtype == PL_F32) PL_ROPE(float);
+    else if (dtype == PL_BF16) PL_ROPE(__nv_bfloat16);
+    else return pl_fail("rope_kv_write: unknown dtype %d", dtype);
+#undef PL_ROPE
     return 0;
 }
 

@@ -650,12 +650,12 @@ class CudaOps:
         return self.act_mul(self.linear(h, w_gate_up), activation)
 
     def qkv_rope_write(self, h, w_qkv, nh, nkv, d, position, ctx, kv, block_table, write=True,
-                       value_from_key=False) -> torch.Tensor:
+                       value_from_key=False, early=False) -> torch.Tensor:
         """The fused q/k/v projection with rotary positions applied to q and k and k, v
         written to the cache.  Returns the [T, (nh + 2 nkv) d] buffer whose first nh*d
         columns are the rotated queries.  `value_from_key`: there is no value projection (w_qkv
         stacks q and k only, the buffer is [T, (nh + nkv) d]) and the value written beside a key
-        is that key as projected, before its rotation."""
+        is that key as projected, before its rotation.  `early`: see `rope_kv_write`."""
         M, K = h.shape
         N = (nh + (1 if value_from_key else 2) * nkv) * d
         assert w_qkv.shape[0] == N
@@ -664,7 +664,7 @@ class CudaOps:
         if not fusable:
             qkv = self.linear(h, w_qkv)
             self.rope_kv_write(qkv, nh, nkv, d, position, ctx, kv, block_table, write=write,
-                               value_from_key=value_from_key)
+                               value_from_key=value_from_key, early=early)
             return qkv
         x, ldx, part, nw, nwc, eps = self._norm_args(h)
         qkv = torch.empty((M, N), dtype=torch.bfloat16, device=self.device)
@@ -1317,9 +1317,11 @@ class CudaOps:
         self.launches += 1
         return table
 
-    def rope_kv_write(self, qkv, nh, nkv, d, position, ctx, kv, block_table, write=True, value_from_key=False, rotated_later=0):
+    def rope_kv_write(self, qkv, nh, nkv, d, position, ctx, kv, block_table, write=True, value_from_key=False, rotated_later=0,
+                      early=False):
         """Rotates the q and k columns of `qkv` in place and writes keys and values to their page slots.  `rotated_later` > 0: the
-        queries of requests that bring more than so many query rows per kv head are left as they are."""
+        queries of requests that bring more than so many query rows per kv head are left as they are.  `early`: the kernels in
+        front, here and behind may overlap at their ends (see the kernel for where that pays)."""
         T = ctx.num_tokens
         assert qkv.is_contiguous() and qkv.shape[0] == T
         if position is not None:
@@ -1333,7 +1335,7 @@ class CudaOps:
             self._p(qkv), self._code(qkv), T, qkv.shape[1], self._p(table), table_len, rd, inter,
             self._p(ctx.positions), self._p(ctx.token_seq), self._p(block_table), block_table.shape[1],
             self._p(kv), num_pages, nh, nkv, d, ps, 1 if write else 0, 1 if value_from_key else 0,
-            self._p(ctx.cu_seqlens_q if rotated_later else None), rotated_later, self._stream))
+            self._p(ctx.cu_seqlens_q if rotated_later else None), rotated_later, 1 if early else 0, self._stream))
         self.launches += 1
 
     # ---- attention ---------------------------------------------------------------
@@ -1437,16 +1439,18 @@ class CudaOps:
         if inside:
             qkv = self.linear(h, w_qkv)
             return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, rope=position, chunk=chunk)
-        if (self.rope_in_attention and plan is not None and plan.n_large and write and softcap is None and slopes is None
-                and position is not None and not value_from_key
-                and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens
-                and not self._skinny_ok(h, (nh + 2 * nkv) * d) and self._prompt_tiles_rotate(nh, nkv, d, kv, position)):
+        tiles = (softcap is None and slopes is None and position is not None and not self._skinny_ok(h, (nh + 2 * nkv) * d)
+                 and self._prompt_tiles_rotate(nh, nkv, d, kv, position))
+        # (then all items run the tensor-core kernels of head sizes 64 and 128 but for small ones of masks and pages these do not take)
+        early = tiles and not window and not chunk and kv.shape[3] % 16 == 0
+        if (self.rope_in_attention and plan is not None and plan.n_large and write and tiles and not value_from_key
+                and position.pairing == "half" and position.rotary_dim == d and M == ctx.num_tokens):
             # the kernel of the prompt tiles rotates the queries it loads
             qkv = self.linear(h, w_qkv)
-            self.rope_kv_write(qkv, nh, nkv, d, position, ctx, kv, block_table, rotated_later=self.SMALL_ROWS)
+            self.rope_kv_write(qkv, nh, nkv, d, position, ctx, kv, block_table, rotated_later=self.SMALL_ROWS, early=early)
             return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, chunk=chunk, tile_rope=position)
         qkv = self.qkv_rope_write(h, w_qkv, nh, nkv, d, position, ctx, kv, block_table, write=write,
-                                  value_from_key=value_from_key)
+                                  value_from_key=value_from_key, early=early)
         return self.paged_attention(qkv, nh, nkv, d, kv, block_table, ctx, scale, window, softcap=softcap, slopes=slopes,
                                     chunk=chunk)
 
