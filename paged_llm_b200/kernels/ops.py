@@ -505,31 +505,38 @@ class CudaOps:
 
     def _gate_up_tc_ok(self, h, w: torch.Tensor, I: int, activation: str) -> bool:
         """Whether the tcgen05 kernel takes the gate/up product.  Below `gemm_tc_min_tokens` its tiles of 256 tokens and 128
-        features, a pair of SMs each, have to fill their waves: the products asked for are 0.75 of what the waves could do, 0.7
-        from the fourth wave on.  us, this kernel and the library's product with `act_mul`:
+        features, a pair of SMs each, have to fill their waves: the products asked for are 0.85 of what the waves could do.  For
+        multiples of 64 tokens (what steps of mixed items are padded to) the library's choice is often slower than for their
+        neighbours (828 and 832 below), and with K up to 2,048 0.75 will do, 0.7 from the fourth wave on.  Below K = 512 a tile's
+        start and end weigh more than the library's, above 4,096 the library's main loop is the faster one.  us, this kernel
+        and the library's product with `act_mul` (* where this one runs):
 
-            tokens    2,048 -> 5,632    2,048 -> 8,192    4,096 -> 14,336
-              256      18.4  15.7        19.7  21.0        57.6  60.7
-              384      27.3  19.1        28.5  26.3        92.6  79.1
-              512      27.4  25.2        28.6  32.1        96.4 107.4
-              576      28.0  27.6        38.3  35.3       120.4 104.8
-              768      28.3  30.9        40.0  45.2       124.5 151.0
-              832      37.7  35.1        50.0  54.9       163.8 167.0
-              960      37.9  36.2        51.3  56.7       189.0 190.1
-            1,024      37.9  43.9        51.9  57.4       185.9 224.6
-            1,408      50.3  57.7        73.6  82.0       249.2 294.8
+            tokens    512 -> 8,192    2,048 -> 5,632    2,048 -> 8,192    4,096 -> 8,192    4,096 -> 14,336
+              512      15.1  18.1 *      27.4  25.9        29.9  33.2 *      55.3  55.6 *      99.3 110.6
+              576      19.3  18.6        28.4  28.2        40.3  37.1        74.8  66.2       127.5 110.6
+              640      19.5  18.8        28.8  30.7        40.8  44.2        76.4  79.2       130.0 155.6
+              700      19.5  21.9        29.3  30.6        41.4  43.8        77.1  78.2       129.5 138.8
+              768      19.5  23.3 *      29.6  32.5 *      42.0  46.7 *      78.5  83.6 *     132.1 142.3 *
+              828      23.7  24.4        38.3  36.3        52.2  50.0        98.7  89.1       167.9 155.3
+              832      23.9  25.2 *      38.0  36.6        52.0  56.3 *      98.0  99.7       164.9 163.8
+              960      24.1  26.1 *      39.1  38.2        53.7  58.4 *      99.7 103.1       169.5 170.0
+            1,024      24.1  30.0 *      39.2  44.5 *      54.3  59.2 *     100.3 104.8 *     170.5 205.8 *
+            1,036      28.3  28.2        42.1  43.3        63.5  60.2       118.8 111.6       197.6 182.3
+            1,085      28.5  29.2        42.4  45.5        64.1  63.3       119.8 111.6       195.6 194.1
+            1,408      33.0  36.9 *      52.8  58.7 *      75.8  84.8 *     141.0 152.9       242.7 270.3
 
-        (The line falls between the sides but for 2,048 -> 5,632 at 640 tokens and 2,048 -> 8,192 at 640, which it leaves to the
-        library: 28.3 against 30.3 and 38.9 against 43.9.  The tanh form of GELU has not been measured below 2,048.)"""
+        Over 7,236 points (K of 64 to 8,192, 1,024 to 14,336 features, 180 to 2,047 tokens, odd numbers among them) it takes 1,654,
+        which take 14 % less time on average and 0.9 % more at worst.  The tanh form of GELU has not been measured below 2,048."""
         if self._gemm_tc_ok(h, w, "silu"):
             return True
         M, K = h.shape
         if not ("silu" in self.gemm_tc_for and activation == "silu" and h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-                and M > 64 and K >= 64 and K % 64 == 0 and w.is_contiguous() and wide(w) and wide(h)):
+                and 512 <= K <= 4096 and K % 64 == 0 and w.is_contiguous() and wide(w) and wide(h)):
             return False
         pairs = self.num_sms // 2
         waves = -(-(-(-M // 256) * -(-I // 128)) // pairs)
-        return M * I >= (0.75 if waves <= 3 else 0.7) * waves * pairs * 256 * 128
+        fill = 0.85 if M % 64 or K > 2048 else 0.75 if waves <= 3 else 0.7
+        return M * I >= fill * waves * pairs * 256 * 128
 
     def _gemm_tc(self, h: torch.Tensor, w: torch.Tensor, out, resid, N: int, epi: int) -> None:
         M, K = h.shape
