@@ -138,7 +138,8 @@ class CudaOps:
         self.mid_widths, self.mid_width_per_token, self.mid_features = (640, 4096), 20, 2 * self.num_sms * 128
         # Many tokens: this package's tcgen05 kernel (pairs of blocks on 256 x 256 tiles, fused epilogues) where it is at least
         # as fast as the library product followed by the elementwise kernel.  Measured: the gate/up product
-        # with SiLU-mul from 2,048 tokens on (65 us against 80 us, timed alone), and below that where its tiles fill the machine
+        # with SiLU-mul from 2,048 tokens on (2,048 -> 5,632: 66 us against 79 one after the other, 77 against 87 with L2 flushed in
+        # between), and below that where its tiles fill the machine
         # (`_gate_up_tc_ok`); the narrower products are faster through the library.  PAGED_LLM_B200_GEMM_TC lists the
         # kinds ("silu", "add", "plain", "all", "" for none) to run on it from 129 tokens on instead.
         tc_for = os.environ.get("PAGED_LLM_B200_GEMM_TC")

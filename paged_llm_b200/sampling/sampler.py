@@ -50,6 +50,7 @@ class Sampler:
         temps = np.array([p.temperature for p in params], np.float32)
         top_k = np.array([p.top_k if p.top_k > 0 else 0 for p in params], np.int32)
         top_p = np.array([p.top_p for p in params], np.float32)
+        # (request_seed's first branch in place: a call each costs 3 us at 64 requests)
         seeds = np.array([request_seed(self.seed, s) if p.seed is None else int(p.seed) & MASK64 for s, p in zip(seqs, params)], np.uint64)
         counters = np.array([len(s.token_ids) for s in seqs], np.uint64)
         return self.ops.sample(logits, temps, top_k, top_p, seeds, counters)
